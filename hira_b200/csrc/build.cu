@@ -456,6 +456,27 @@ __global__ void scatter_gps_kernel(const T* __restrict__ cents2, const int32_t* 
     if (ch == 0) gp_counts[(size_t)h * cap_gp + g] = fill2[(size_t)h * k2 + g];
 }
 
+// Child slots that hold no key: zero rows, token -1.  One warp per parent; the free slots of a parent
+// are its last ones, so they are one run of whole 16-byte pieces per array.
+constexpr int UNFILLED_THREADS = 256;
+__global__ void __launch_bounds__(UNFILLED_THREADS)
+clear_unfilled_kernel(const int32_t* __restrict__ child_counts, int cap_parents, int n_parents, int bf,
+                      uint4* __restrict__ children, int row_pieces, uint4* __restrict__ values, int vrow_pieces,
+                      int32_t* __restrict__ slot2token) {
+    const int p = blockIdx.x * (UNFILLED_THREADS / 32) + (threadIdx.x >> 5), wl = threadIdx.x & 31;
+    if (p >= n_parents) return;
+    const size_t hp = (size_t)blockIdx.y * cap_parents + p;
+    const int cnt = child_counts[hp];
+    if (cnt >= bf) return;
+    const size_t slot = hp * bf + cnt;
+    const int n = bf - cnt;
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = wl; i < n * row_pieces; i += 32) children[slot * row_pieces + i] = z;
+    for (int i = wl; i < n * vrow_pieces; i += 32) values[slot * vrow_pieces + i] = z;
+    if (slot2token)
+        for (int i = wl; i < n; i += 32) slot2token[slot + i] = -1;
+}
+
 __global__ void set_used_kernel(int32_t* used, int n_heads, int used_p, int used_g, int n_keys) {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= n_heads) return;
@@ -708,37 +729,50 @@ static int build_impl(const hira_index_t* ix, const void* keys_v, const void* va
     const size_t capP = ix->cap_parents, capC = capP * bf;
     // ---- clear the index -----------------------------------------------------
     // Everything, or -- when the host vouches through active_parents that no slot beyond that bound
-    // was ever used -- the slots up to the larger of that bound and what this build fills.
+    // was ever used -- the slots up to the larger of that bound and what this build fills.  The child
+    // rows, the bulk of the index, are not cleared here: the scatter below writes the filled ones and
+    // clear_unfilled_kernel the rest, each once.
+    size_t clearP = capP;
+    if (ix->active_parents > 0) {
+        const size_t fills = ix->depth == 3 ? (size_t)k2 * bf : (size_t)k1;
+        clearP = (size_t)ix->active_parents > fills ? (size_t)ix->active_parents : fills;
+        if (clearP > capP) clearP = capP;
+    }
     {
-        size_t clearP = capP;
-        if (ix->active_parents > 0) {
-            const size_t fills = ix->depth == 3 ? (size_t)k2 * bf : (size_t)k1;
-            clearP = (size_t)ix->active_parents > fills ? (size_t)ix->active_parents : fills;
-            if (clearP > capP) clearP = capP;
-        }
-        const size_t clearC = clearP * bf, clearG = ix->depth == 3 ? (clearP + bf - 1) / bf : 0;
+        const size_t clearG = ix->depth == 3 ? (clearP + bf - 1) / bf : 0;
         auto clear = [&](void* ptr, int value, size_t row_bytes, size_t rows_cap, size_t rows_clear) {
             if (ptr) cudaMemset2DAsync(ptr, rows_cap * row_bytes, value, rows_clear * row_bytes, (size_t)H, s);
         };
-        clear(ix->children, 0, dim * es, capC, clearC);
-        clear(ix->values, 0, ix->values ? ix->vdim * elem_size(ix->vdtype) : 0, capC, clearC);
-        clear(ix->slot2token, 0xff, 4, capC, clearC);
         clear(ix->parents, 0, dim * es, capP, clearP);
-        clear(ix->parent_radii, 0, 4, capP, clearP);
-        clear(ix->parent_sqnorm, 0, 4, capP, clearP);
         clear(ix->child_counts, 0, 4, capP, clearP);
         if (ix->depth == 3) {
             clear(ix->grand_parents, 0, dim * es, ix->cap_gp, clearG);
-            clear(ix->gp_radii, 0, 4, ix->cap_gp, clearG);
-            clear(ix->gp_sqnorm, 0, 4, ix->cap_gp, clearG);
             clear(ix->gp_counts, 0, 4, ix->cap_gp, clearG);
+        }
+        if (n_keys == 0) {   // otherwise written by the radii kernels
+            clear(ix->parent_radii, 0, 4, capP, clearP);
+            clear(ix->parent_sqnorm, 0, 4, capP, clearP);
+            if (ix->depth == 3) {
+                clear(ix->gp_radii, 0, 4, ix->cap_gp, clearG);
+                clear(ix->gp_sqnorm, 0, 4, ix->cap_gp, clearG);
+            }
         }
     }
     HIRA_CHECK_LAUNCH("index clear");
+    auto clear_unfilled = [&]() -> int {
+        const int warps = UNFILLED_THREADS / 32;
+        dim3 grid((unsigned)((clearP + warps - 1) / warps), (unsigned)H);
+        clear_unfilled_kernel<<<grid, UNFILLED_THREADS, 0, s>>>(
+            ix->child_counts, (int)capP, (int)clearP, bf, reinterpret_cast<uint4*>(ix->children), (int)(dim * es / 16),
+            reinterpret_cast<uint4*>(ix->values), ix->values ? (int)(ix->vdim * elem_size(ix->vdtype) / 16) : 0,
+            ix->slot2token);
+        HIRA_CHECK_LAUNCH("clear unfilled launch");
+        return HIRA_OK;
+    };
     if (n_keys == 0) {
         set_used_kernel<<<(H + 127) / 128, 128, 0, s>>>(ix->used, H, 0, 0, 0);
         HIRA_CHECK_LAUNCH("set used launch");
-        return HIRA_OK;
+        return clear_unfilled();
     }
     T* cents1 = reinterpret_cast<T*>(base + w.cents1);
     T* cents2 = reinterpret_cast<T*>(base + w.cents2);
@@ -788,6 +822,8 @@ static int build_impl(const hira_index_t* ix, const void* keys_v, const void* va
                                                              nullptr, 0);
         HIRA_CHECK_LAUNCH("scatter values launch");
     }
+    rc = clear_unfilled();
+    if (rc != HIRA_OK) return rc;
     set_used_kernel<<<(H + 127) / 128, 128, 0, s>>>(ix->used, H, ix->depth == 3 ? k2 * bf : k1,
                                                      ix->depth == 3 ? k2 : 0, n_keys);
     HIRA_CHECK_LAUNCH("set used launch");

@@ -18,7 +18,9 @@ from . import _lib as L
 class IndexState:
     def __init__(self, *, n_heads: int, dim: int, vdim: int, bf: int, depth: int, cap_parents: int,
                  dtype: torch.dtype, vdtype: Optional[torch.dtype], device, with_values: bool = True,
-                 int8_copy: Optional[bool] = None):
+                 int8_copy: Optional[bool] = None, cleared: bool = True):
+        """`cleared=False`: for a state that `build` fills with at least one key next -- the build writes
+        every array (keys, or zeros and -1 where there are none), so nothing is cleared here first."""
         if depth not in (2, 3):
             raise ValueError(f"Unsupported depth {depth}")
         self.n_heads, self.dim, self.vdim, self.bf, self.depth = n_heads, dim, vdim if with_values else 0, bf, depth
@@ -32,10 +34,12 @@ class IndexState:
             self.cap_parents = max(1, cap_parents)
         capC = self.cap_parents * bf
         dev = self.device
-        z = torch.zeros
+        z = torch.zeros if cleared else torch.empty
         self.children = z((n_heads, capC, dim), dtype=dtype, device=dev)
         self.values = z((n_heads, capC, self.vdim), dtype=self.vdtype, device=dev) if with_values else None
-        self.slot2token = torch.full((n_heads, capC), -1, dtype=torch.int32, device=dev)
+        self.slot2token = z((n_heads, capC), dtype=torch.int32, device=dev)
+        if cleared:
+            self.slot2token.fill_(-1)
         self.parents = z((n_heads, self.cap_parents, dim), dtype=dtype, device=dev)
         self.parent_radii = z((n_heads, self.cap_parents), dtype=torch.float32, device=dev)
         self.parent_sqnorm = z((n_heads, self.cap_parents), dtype=torch.float32, device=dev)
@@ -58,7 +62,9 @@ class IndexState:
         if self.int8_copy:
             self.children_q8 = z((n_heads, capC, 128), dtype=torch.int8, device=dev)
             self.children_q8_meta = z((n_heads, capC), dtype=torch.int32, device=dev)   # (step, error bound) as two fp16
-            self.q8_chan_scale = torch.ones((n_heads, L.Q8_CHAN), dtype=torch.float32, device=dev)
+            self.q8_chan_scale = z((n_heads, L.Q8_CHAN), dtype=torch.float32, device=dev)
+            if cleared:
+                self.q8_chan_scale.fill_(1.0)
             self.q8_query_scratch = z((n_heads, L.Q8_QUERY_BYTES), dtype=torch.uint8, device=dev)
         else:
             self.children_q8 = self.children_q8_meta = self.q8_chan_scale = self.q8_query_scratch = None

@@ -187,7 +187,7 @@ class CUDAIndexer(BaseIndexer):
         if st is None:
             st = S.IndexState(n_heads=h, dim=d, vdim=vdim, bf=bf, depth=self.depth.value, cap_parents=cap_p,
                               dtype=keys.dtype, vdtype=values.dtype if values is not None else None, device=keys.device,
-                              with_values=values is not None)
+                              with_values=values is not None, cleared=n == 0)
         else:
             st.active_parents = self.active_parents     # the build clears only what was in use
         k1 = -(-n // bf) if n else 0

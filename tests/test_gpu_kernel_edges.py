@@ -35,3 +35,29 @@ def test_threshold_sorts_nan_scores_last():
     keep = torch.cat([samples[:, :17], samples[:, 18:]], dim=1).contiguous()
     for k in (5, 40):
         assert torch.equal(S.threshold(samples, q, L.HIRA_TAU_SAMPLE_MEAN_TOPK, k), S.threshold(keep, q, L.HIRA_TAU_SAMPLE_MEAN_TOPK, k))
+
+
+@pytest.mark.parametrize("depth,bf,n,spare,vals,dtype", [
+    (3, 8, 1000, 300, True, torch.bfloat16), (3, 8, 1, 0, True, torch.float32), (2, 16, 1001, 64, True, torch.float32),
+    (2, 1, 37, 5, False, torch.bfloat16), (3, 32, 4096, 0, False, torch.bfloat16)])
+def test_build_into_dirty_memory_leaves_free_slots_clear(depth, bf, n, spare, vals, dtype):
+    """A state that was not cleared before its build is, bit for bit, one that was; so is a rebuild in place."""
+    h, d = 3, 64
+    keys = make_keys(h, n, d, 1, dtype)
+    values = make_keys(h, n, d, 2, dtype) if vals else None
+    k1 = -(-n // bf)
+    cap = (-(-k1 // bf) * bf if depth == 3 else k1) + spare
+    kw = dict(n_heads=h, dim=d, vdim=d, bf=bf, depth=depth, cap_parents=cap, dtype=dtype, vdtype=dtype, device="cuda", with_values=vals)
+    ref = S.IndexState(**kw)
+    S.build(ref, keys, values)
+    st = S.IndexState(**kw, cleared=False)
+    for name in S.IndexState.ARRAYS + S.IndexState.Q8_ARRAYS:
+        t = getattr(st, name)
+        if t is not None:
+            t.view(torch.uint8).fill_(0x5A)
+    for again in range(2):
+        S.build(st, keys, values)
+        for name in S.IndexState.ARRAYS:
+            a, b = getattr(ref, name), getattr(st, name)
+            if a is not None:
+                assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)), (name, again)
