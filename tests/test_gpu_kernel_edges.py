@@ -61,3 +61,11 @@ def test_build_into_dirty_memory_leaves_free_slots_clear(depth, bf, n, spare, va
             a, b = getattr(ref, name), getattr(st, name)
             if a is not None:
                 assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)), (name, again)
+
+
+@pytest.mark.parametrize("n,d,bf,dtype", [(700, 8, 4, torch.bfloat16), (700, 72, 64, torch.float32), (65, 128, 64, torch.bfloat16),
+                                          (1500, 200, 100, torch.bfloat16), (97, 256, 97, torch.float32)])
+def test_lloyd_means_match_oracle(n, d, bf, dtype):
+    """Clusters of fewer, exactly and more members than a batch of rows in flight; channels that are no whole slab."""
+    st, ox, _, _ = build_both(2, n, d, bf, 2, dtype, seed=5, n_iters=3)
+    assert_index_equal(st, ox, "lloyd")
