@@ -69,3 +69,20 @@ def test_lloyd_means_match_oracle(n, d, bf, dtype):
     """Clusters of fewer, exactly and more members than a batch of rows in flight; channels that are no whole slab."""
     st, ox, _, _ = build_both(2, n, d, bf, 2, dtype, seed=5, n_iters=3)
     assert_index_equal(st, ox, "lloyd")
+
+
+@pytest.mark.parametrize("n_parts,vdim,hq", [(1, 8, 1), (15, 128, 5), (16, 136, 3), (17, 256, 2), (64, 128, 4), (65, 40, 3), (200, 300, 2)])
+def test_merge_partials_edges(n_parts, vdim, hq):
+    """Batches of rows in flight, weights staged 64 at a time, more channels than threads; some parts empty."""
+    g = torch.Generator().manual_seed(n_parts)
+    o = torch.randn((n_parts, hq, vdim), generator=g)
+    ml = torch.stack([torch.randn((n_parts, hq), generator=g) * 5, torch.rand((n_parts, hq), generator=g) + 0.1], dim=-1)
+    if n_parts > 2:
+        ml[1, 0, 0], ml[1, 0, 1], o[1, 0] = float("-inf"), 0.0, 0.0
+    out_ml = torch.empty((hq, 2), device="cuda")
+    got = S.merge_partials(o.cuda(), ml.cuda(), out_ml=out_ml).cpu().double()
+    w = torch.exp(ml[..., 0].double() - ml[..., 0].double().max(dim=0).values) * ml[..., 1].double()
+    want = (w[..., None] * o.double()).sum(0) / w.sum(0)[:, None]
+    # weights by __expf (2 ulp + 2^-21 |x|, |x| <= 40) and fp32 sums of n_parts terms
+    assert (got - want).norm() / want.norm() < 4e-6 + n_parts * 6e-8
+    assert torch.equal(out_ml[:, 0].cpu(), ml[..., 0].max(dim=0).values)
