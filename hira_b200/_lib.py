@@ -26,6 +26,7 @@ EXPORTED_SYMBOLS = [
     "hira_append_workspace_bytes",
     "hira_threshold", "hira_kth_score", "hira_prepare_query", "hira_build_workspace_bytes", "hira_build",
     "hira_recompute_radii", "hira_export", "hira_assign", "hira_sparse_attn_noalloc", "hira_decode_attention",
+    "hira_decode_attention_sampled",
     "hira_search_scan", "hira_append_scanned", "hira_step_events_create", "hira_step_events_destroy",
     "hira_decode_step", "hira_q8_refresh", "hira_q8_fallback_count",
     "hira_exchange_bytes", "hira_peer_alloc", "hira_peer_open", "hira_peer_close", "hira_peer_free", "hira_exchange_merge",
@@ -88,6 +89,9 @@ def _declare(lib):
     lib.hira_decode_attention.restype = C.c_int
     lib.hira_decode_attention.argtypes = [IX, P, I32, C.c_float, P, P, I32, I32, I32, I32, P, P, P, P, P, P, P, I32, I64,
                                           I32, P, P, P, I64, I64, P, I64, P, P, P]
+    lib.hira_decode_attention_sampled.restype = C.c_int
+    lib.hira_decode_attention_sampled.argtypes = [IX, P, I32, C.c_float, P, I32, I64, I32, I32, P, P, I32, I32, I32, I32, P, P,
+                                                  P, P, P, P, P, I32, I64, I32, P, P, P, I64, I64, P, I64, P, P, P]
     ST = C.POINTER(HiraStepStruct)
     lib.hira_step_events_create.restype = C.c_int
     lib.hira_step_events_create.argtypes = [ST]

@@ -20,8 +20,13 @@ import torch
 
 from .. import _lib as L
 from .. import index_state as S
-from ..cache.threshold_finder import THRESHOLD_METHODS
+from ..cache.threshold_finder import THRESHOLD_METHODS, sample_kth, sample_max, sample_mean_topk
 from ..searcher import CUDASearcher
+
+
+# the library's own finders: their threshold is found inside the one call of a decode step
+_FINDERS = {"sample_max": (sample_max, L.HIRA_TAU_SAMPLE_MAX), "sample_mean_topk": (sample_mean_topk, L.HIRA_TAU_SAMPLE_MEAN_TOPK),
+            "sample_kth": (sample_kth, L.HIRA_TAU_SAMPLE_KTH)}
 
 
 def _samples_for(indexer, sample_size: int) -> torch.Tensor:
@@ -110,16 +115,21 @@ def hira_decode_attention(query: torch.Tensor, cache_output, *, scaling: Optiona
         if q2kv is not None:
             raise ValueError("append_key needs the default query-head grouping")
         scan_key, scan_out = indexer.begin_scanned_update(append_key)
-    if threshold is not None and threshold_method != "none":
-        # the usual decode step: the threshold is known, one library call does the rest
-        tau = threshold
+    finder = {}
+    if threshold is None and threshold_method in _FINDERS and THRESHOLD_METHODS[threshold_method] is _FINDERS[threshold_method][0]:
+        samples = _samples_for(indexer, sample_size)
+        finder = dict(tau_samples=samples, tau_method=_FINDERS[threshold_method][1],
+                      tau_k=1 if threshold_method == "sample_max" else min(int(topk), samples.shape[1]))
+    if finder or (threshold is not None and threshold_method != "none"):
+        # the threshold is known or found from the index's samples: one library call does the rest
+        tau = torch.empty((n_q,), dtype=torch.float32, device=st.device) if finder else threshold
         if tau.shape != (n_q,):
             raise ValueError(f"threshold must have shape ({n_q},), got {tuple(tau.shape)}")
         if tau.device != st.device or tau.dtype != torch.float32 or not tau.is_contiguous():
             tau = tau.to(device=st.device, dtype=torch.float32).contiguous()
         S.decode_attention(st, q, sm_scale, tau, compact, bufs[0], bufs[1], q2kv=q2kv, max_group=max_group,
                            flags=srch.flags, queued_k=queued_k, queued_v=queued_v, n_splits=n_splits, workspace=ws,
-                           out=out, scan_key=scan_key, scan_out=scan_out,
+                           out=out, scan_key=scan_key, scan_out=scan_out, **finder,
                            searched_event=indexer.searched_event() if hasattr(indexer, "searched_event") else None)
     else:
         q_hat, logit_scale = S.prepare_query(q, sm_scale, bufs[0], bufs[1])

@@ -1,5 +1,6 @@
 // Error plumbing and argument validation shared by every entry point.
 #include "common.cuh"
+#include "search_common.cuh"
 
 #include <stdarg.h>
 #include <string.h>
@@ -64,6 +65,35 @@ int validate_index(const hira_index_t* ix, bool need_values) {
 extern "C" const char* hira_last_error(void) { return hira::g_err; }
 extern "C" const char* hira_version(void) { return "hira_b200 0.1 (sm_100a)"; }
 
+namespace {
+int decode_attention(const hira_index_t* index, const hira::RawQuery& raw, const hira::TauFinder* finder, const float* tau,
+                     const int32_t* q2kv, int32_t n_qheads, int32_t max_group, int32_t flags, int32_t tile_parents,
+                     int32_t* idx, float* score, int32_t* count, const void* queued_k, const void* queued_v,
+                     int32_t n_queued, int64_t queued_head_stride, int32_t n_splits, float* workspace, float* out,
+                     float* out_ml, int64_t out_head_stride, int64_t ml_head_stride, const void* scan_key,
+                     int64_t scan_key_stride, uint64_t* scan_out, void* searched, void* stream) {
+    HIRA_CHECK_ARG(index != nullptr, HIRA_ERR_ARG, "hira_decode_attention: index is NULL");
+    HIRA_CHECK_ARG(raw.q && raw.q_hat && raw.logit_scale, HIRA_ERR_ARG,
+                   "hira_decode_attention: q, q_hat and logit_scale must not be NULL");
+    HIRA_CHECK_ARG(scan_out == nullptr || q2kv == nullptr, HIRA_ERR_ARG,
+                   "hira_decode_attention: the fused parent scan needs q2kv == NULL");
+    int rc = hira::query_and_search(index, raw, finder, tau, q2kv, n_qheads, max_group, flags, tile_parents, idx, score,
+                                    count, scan_key, scan_key_stride, reinterpret_cast<unsigned long long*>(scan_out),
+                                    reinterpret_cast<cudaStream_t>(stream));
+    if (rc != HIRA_OK) return rc;
+    if (searched != nullptr) {
+        cudaError_t e = cudaEventRecord(reinterpret_cast<cudaEvent_t>(searched), reinterpret_cast<cudaStream_t>(stream));
+        if (e != cudaSuccess) {
+            hira::set_error("hira_decode_attention: cudaEventRecord: %s", cudaGetErrorString(e));
+            return HIRA_ERR_CUDA;
+        }
+    }
+    return hira_sparse_attn(index, raw.q_hat, raw.logit_scale, q2kv, n_qheads, tile_parents, idx, score, count,
+                            queued_k, queued_v, n_queued, queued_head_stride, n_splits, workspace, out, out_ml,
+                            out_head_stride, ml_head_stride, stream);
+}
+}  // namespace
+
 extern "C" int hira_decode_attention(const hira_index_t* index, const void* q, int32_t q_dtype, float sm_scale,
                                      const float* tau, const int32_t* q2kv, int32_t n_qheads, int32_t max_group,
                                      int32_t flags, int32_t tile_parents, float* q_hat, float* logit_scale,
@@ -73,29 +103,29 @@ extern "C" int hira_decode_attention(const hira_index_t* index, const void* q, i
                                      float* out, float* out_ml, int64_t out_head_stride, int64_t ml_head_stride,
                                      const void* scan_key, int64_t scan_key_stride, uint64_t* scan_out,
                                      void* searched, void* stream) {
-    HIRA_CHECK_ARG(index != nullptr, HIRA_ERR_ARG, "hira_decode_attention: index is NULL");
-    HIRA_CHECK_ARG(q && q_hat && logit_scale, HIRA_ERR_ARG, "hira_decode_attention: q, q_hat and logit_scale must not be NULL");
-    int rc = hira_prepare_query(q, q_dtype, n_qheads, index->dim, sm_scale, q_hat, logit_scale, stream);
-    if (rc != HIRA_OK) return rc;
-    if (scan_out != nullptr) {
-        HIRA_CHECK_ARG(q2kv == nullptr, HIRA_ERR_ARG, "hira_decode_attention: the fused parent scan needs q2kv == NULL");
-        rc = hira_search_scan(index, q_hat, tau, logit_scale, nullptr, n_qheads, flags, tile_parents, nullptr, idx,
-                              score, count, nullptr, scan_key, scan_key_stride, scan_out, stream);
-    } else {
-        rc = hira_search(index, q_hat, tau, logit_scale, nullptr, q2kv, n_qheads, max_group, flags, tile_parents,
-                         nullptr, idx, score, count, nullptr, stream);
-    }
-    if (rc != HIRA_OK) return rc;
-    if (searched != nullptr) {
-        cudaError_t e = cudaEventRecord(reinterpret_cast<cudaEvent_t>(searched), reinterpret_cast<cudaStream_t>(stream));
-        if (e != cudaSuccess) {
-            hira::set_error("hira_decode_attention: cudaEventRecord: %s", cudaGetErrorString(e));
-            return HIRA_ERR_CUDA;
-        }
-    }
-    return hira_sparse_attn(index, q_hat, logit_scale, q2kv, n_qheads, tile_parents, idx, score, count,
+    const hira::RawQuery raw{q, q_dtype, sm_scale, q_hat, logit_scale};
+    return decode_attention(index, raw, nullptr, tau, q2kv, n_qheads, max_group, flags, tile_parents, idx, score, count,
                             queued_k, queued_v, n_queued, queued_head_stride, n_splits, workspace, out, out_ml,
-                            out_head_stride, ml_head_stride, stream);
+                            out_head_stride, ml_head_stride, scan_key, scan_key_stride, scan_out, searched, stream);
+}
+
+extern "C" int hira_decode_attention_sampled(const hira_index_t* index, const void* q, int32_t q_dtype, float sm_scale,
+                                             const void* tau_samples, int32_t n_samples, int64_t samples_head_stride,
+                                             int32_t tau_method, int32_t tau_k, float* tau,
+                                             const int32_t* q2kv, int32_t n_qheads, int32_t max_group,
+                                             int32_t flags, int32_t tile_parents, float* q_hat, float* logit_scale,
+                                             int32_t* idx, float* score, int32_t* count,
+                                             const void* queued_k, const void* queued_v, int32_t n_queued,
+                                             int64_t queued_head_stride, int32_t n_splits, float* workspace,
+                                             float* out, float* out_ml, int64_t out_head_stride, int64_t ml_head_stride,
+                                             const void* scan_key, int64_t scan_key_stride, uint64_t* scan_out,
+                                             void* searched, void* stream) {
+    HIRA_CHECK_ARG(tau_samples && tau, HIRA_ERR_ARG, "hira_decode_attention_sampled: tau_samples and tau must not be NULL");
+    const hira::RawQuery raw{q, q_dtype, sm_scale, q_hat, logit_scale};
+    const hira::TauFinder finder{tau_samples, n_samples, samples_head_stride, tau_method, tau_k, tau};
+    return decode_attention(index, raw, &finder, nullptr, q2kv, n_qheads, max_group, flags, tile_parents, idx, score, count,
+                            queued_k, queued_v, n_queued, queued_head_stride, n_splits, workspace, out, out_ml,
+                            out_head_stride, ml_head_stride, scan_key, scan_key_stride, scan_out, searched, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -181,22 +211,11 @@ extern "C" int hira_decode_step(const hira_index_t* index, const hira_step_t* st
             HIRA_CUDA_OK(cudaStreamWaitEvent(main_s, copied, 0), "stream wait");
         }
     }
-    rc = hira_prepare_query(st->q_dev, q_dtype, n_qheads, index->dim, sm_scale, st->q_hat, st->logit_scale, stream);
-    if (rc != HIRA_OK) return rc;
-    const float* tau = tau_dev;
-    if (tau == nullptr) {
-        rc = hira_threshold(st->tau_samples, index->dtype, index->n_heads, st->n_samples, index->dim,
-                            st->samples_head_stride, st->q_hat, nullptr, n_qheads, st->tau_method, st->tau_k, st->tau,
-                            stream);
-        if (rc != HIRA_OK) return rc;
-        tau = st->tau;
-    }
-    if (fused)
-        rc = hira_search_scan(index, st->q_hat, tau, st->logit_scale, nullptr, n_qheads, st->flags, st->tile_parents,
-                              nullptr, st->idx, st->score, st->count, nullptr, st->k_dev, index->dim, st->scan, stream);
-    else
-        rc = hira_search(index, st->q_hat, tau, st->logit_scale, nullptr, nullptr, n_qheads, 0, st->flags,
-                         st->tile_parents, nullptr, st->idx, st->score, st->count, nullptr, stream);
+    const hira::RawQuery raw{st->q_dev, q_dtype, sm_scale, st->q_hat, st->logit_scale};
+    const hira::TauFinder finder{st->tau_samples, st->n_samples, st->samples_head_stride, st->tau_method, st->tau_k, st->tau};
+    rc = hira::query_and_search(index, raw, tau_dev ? nullptr : &finder, tau_dev, nullptr, n_qheads, 0, st->flags,
+                                st->tile_parents, st->idx, st->score, st->count, fused ? st->k_dev : nullptr, index->dim,
+                                fused ? reinterpret_cast<unsigned long long*>(st->scan) : nullptr, main_s);
     if (rc != HIRA_OK) return rc;
     if (append) {
         // the attention reads nothing the append writes: the append only waits for the search

@@ -86,6 +86,8 @@ sparse_attn_kernel(const AttnParams P) {
     extern __shared__ __align__(16) float s_out[];  // [ATTN_HW][vdim] at the end; the gather ring before
     using Ring = GatherRing<TV, NVCH>;
 
+    grid_wait();
+    grid_trigger();
     const int tid = threadIdx.x;
     const int lane = tid & (GROUP - 1);
     const int hw = tid / GROUP;
@@ -358,6 +360,7 @@ __global__ void merge_kernel(const float* __restrict__ part_o, const float* __re
                              long long ml_part_stride, long long ml_head_stride,
                              int n_parts, int vdim, int normalised, float* __restrict__ out,
                              float* __restrict__ out_ml, long long out_stride, long long out_ml_stride) {
+    grid_wait();
     const int qh = blockIdx.x;
     merge_row(part_o + qh * o_head_stride, part_ml + qh * ml_head_stride, o_part_stride, ml_part_stride, n_parts, vdim,
               normalised, out + (size_t)qh * out_stride, out_ml ? out_ml + (size_t)qh * out_ml_stride : nullptr);
@@ -376,8 +379,11 @@ static int launch_attn_n(const AttnParams& P, cudaStream_t s) {
             return HIRA_ERR_CUDA;
         }
     }
-    kern<<<grid, ATTN_THREADS, smem, s>>>(P);
-    HIRA_CHECK_LAUNCH("hira_sparse_attn launch");
+    const cudaError_t e = launch_chained(kern, grid, dim3(ATTN_THREADS), smem, s, P);
+    if (e != cudaSuccess) {
+        set_error("hira_sparse_attn launch: %s", cudaGetErrorString(e));
+        return HIRA_ERR_CUDA;
+    }
     return HIRA_OK;
 }
 
@@ -459,10 +465,14 @@ extern "C" int hira_sparse_attn(const hira_index_t* ix, const float* q, const fl
     if (rc != HIRA_OK) return rc;
     if (n_splits == 1) return HIRA_OK;  // the attention kernel wrote `out` itself
     const long long pstride = ix->vdim + 2;
-    merge_kernel<<<n_qheads, 128, 0, s>>>(workspace + 2, workspace, pstride, pstride * n_splits, pstride,
-                                          pstride * n_splits, n_splits, ix->vdim, 0, out, out_ml, P.out_stride,
-                                          P.ml_stride);
-    HIRA_CHECK_LAUNCH("hira_sparse_attn merge launch");
+    const cudaError_t e = launch_chained(merge_kernel, dim3((unsigned)n_qheads), dim3(128), 0, s,
+                                         (const float*)(workspace + 2), (const float*)workspace, pstride, pstride * n_splits,
+                                         pstride, pstride * n_splits, n_splits, (int)ix->vdim, 0, out, out_ml, P.out_stride,
+                                         P.ml_stride);
+    if (e != cudaSuccess) {
+        set_error("hira_sparse_attn merge launch: %s", cudaGetErrorString(e));
+        return HIRA_ERR_CUDA;
+    }
     return HIRA_OK;
 }
 

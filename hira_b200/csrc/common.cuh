@@ -48,6 +48,29 @@ void set_error(const char* fmt, ...);
     } while (0)
 
 int validate_index(const hira_index_t* ix, bool need_values);
+
+// Programmatic launches.  The kernels of one decode step follow each other on one stream; launched with
+// launch_chained, a kernel's CTAs may become resident while the kernel before it still runs, so that the
+// launch latency and the prologue are not on the step's critical path.  A kernel launched so calls
+// grid_wait() before it touches anything an earlier kernel writes (it returns when the kernel before it is
+// complete, and is a no-op after a plain launch), and grid_trigger() only after that, which keeps the
+// order transitive over the whole chain.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename K, typename... A>
+inline cudaError_t launch_chained(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
 // tiles of `tile_parents` parent slots that can hold keys (hira_index_t::active_parents)
 int active_tiles(const hira_index_t* ix, int tile_parents);
 

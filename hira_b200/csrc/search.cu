@@ -102,25 +102,6 @@ search_kernel(const SearchParams P) {
     const int g0 = P.tile_gp_shift >= 0 ? (tile >> P.tile_gp_shift)
                                         : (P.tile_gp_shift == -1 ? tile * P.ng : div_bf(tile * TP, bf, P.bf_magic));
     const int ng = P.ng;
-    int my_qh = qh_of[0];
-#pragma unroll
-    for (int j = 1; j < GT; ++j)
-        if (my_head == j) my_qh = qh_of[j];
-    const float my_tau = head_on ? P.tau[my_qh] : 0.f;
-    const float my_qn = (head_on && has_qn) ? P.qnorm[my_qh] : 1.f;
-    if (tid < nq) s_scale[tid] = P.scaling ? P.scaling[s_qh[tid]] : 1.0f;  // s_qh[tid] was written by this thread or before the barrier above
-    float qreg[GT][NCH][8];
-#pragma unroll
-    for (int j = 0; j < GT; ++j) {
-        if (j < nq) {
-            load_vec_f32<NCH>(P.q + (size_t)qh_of[j] * P.dim, qreg[j], lane, P.dim);
-        } else {
-#pragma unroll
-            for (int i = 0; i < NCH; ++i)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) qreg[j][i][e] = 0.f;
-        }
-    }
     // grandparent row of this group (first pass of the loop below) and its radius
     RawChunk<T> graw[NCH];
     float grad = 0.f;
@@ -143,6 +124,27 @@ search_kernel(const SearchParams P) {
         prad[u] = in ? P.parent_radii[(size_t)h * P.cap_parents + p] : 0.f;
         pcnt[u] = in ? P.child_counts[(size_t)h * P.cap_parents + p] : 0;
         pgc[u] = (in && P.depth == 3) ? P.gp_counts[(size_t)h * P.cap_gp + g0 + div_bf(p - g0 * bf, bf, P.bf_magic)] : 0;
+    }
+    if (P.chained) grid_wait();   // the index is at rest; the query, its threshold and scale may still be on their way
+    grid_trigger();
+    int my_qh = qh_of[0];
+#pragma unroll
+    for (int j = 1; j < GT; ++j)
+        if (my_head == j) my_qh = qh_of[j];
+    const float my_tau = head_on ? P.tau[my_qh] : 0.f;
+    const float my_qn = (head_on && has_qn) ? P.qnorm[my_qh] : 1.f;
+    if (tid < nq) s_scale[tid] = P.scaling ? P.scaling[s_qh[tid]] : 1.0f;  // s_qh[tid] was written by this thread or before the barrier above
+    float qreg[GT][NCH][8];
+#pragma unroll
+    for (int j = 0; j < GT; ++j) {
+        if (j < nq) {
+            load_vec_f32<NCH>(P.q + (size_t)qh_of[j] * P.dim, qreg[j], lane, P.dim);
+        } else {
+#pragma unroll
+            for (int i = 0; i < NCH; ++i)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) qreg[j][i][e] = 0.f;
+        }
     }
     // the new key of this head and the cached squared norms of the same parents, for the scan
     const bool do_scan = SCAN && chunk == 0;  // SCAN: the launch was given a scan_out
@@ -660,6 +662,14 @@ static int launch_search_sc(SearchParams P, int chunks, cudaStream_t stream) {
     HIRA_CHECK_ARG(P.n_tiles <= 65535 && P.n_heads <= 65535, HIRA_ERR_SHAPE,
                    "hira_search: %d tiles x %d heads exceed the grid limits", P.n_tiles, P.n_heads);
     dim3 grid((unsigned)chunks, (unsigned)P.n_tiles_active, (unsigned)P.n_heads);
+    if (P.chained) {
+        const cudaError_t e = launch_chained(kern, grid, dim3(SEARCH_THREADS), smem, stream, P);
+        if (e != cudaSuccess) {
+            set_error("hira_search launch: %s", cudaGetErrorString(e));
+            return HIRA_ERR_CUDA;
+        }
+        return HIRA_OK;
+    }
     kern<<<grid, SEARCH_THREADS, smem, stream>>>(P);
     HIRA_CHECK_LAUNCH("hira_search launch");
     return HIRA_OK;
@@ -723,12 +733,13 @@ extern "C" int hira_search_tile_parents(const hira_index_t* ix) {
     return tp;
 }
 
-static int search_impl(const hira_index_t* ix, const float* q, const float* tau,
-                       const float* scaling, const float* qnorm, const int32_t* q2kv,
-                       int32_t n_qheads, int32_t max_group, int32_t flags,
-                       int32_t tile_parents, float* out_dense, int32_t* out_idx,
-                       float* out_score, int32_t* out_count, uint32_t* stats,
-                       const void* scan_key, int64_t scan_key_stride, unsigned long long* scan_out, void* stream) {
+// checks the arguments of a search and fills its launch parameters
+static int search_setup(const hira_index_t* ix, const float* q, const float* tau,
+                        const float* scaling, const float* qnorm, const int32_t* q2kv,
+                        int32_t n_qheads, int32_t& max_group, int32_t flags,
+                        int32_t tile_parents, float* out_dense, int32_t* out_idx,
+                        float* out_score, int32_t* out_count, uint32_t* stats,
+                        const void* scan_key, int64_t scan_key_stride, unsigned long long* scan_out, SearchParams& P) {
     int rc = validate_index(ix, false);
     if (rc != HIRA_OK) return rc;
     if (scan_out != nullptr) {
@@ -761,7 +772,6 @@ static int search_impl(const hira_index_t* ix, const float* q, const float* tau,
         group = 0;
         if (max_group <= 0 || max_group > n_qheads) max_group = n_qheads;
     }
-    SearchParams P;
     P.children = ix->children; P.parents = ix->parents; P.gps = ix->grand_parents;
     P.parent_radii = ix->parent_radii; P.gp_radii = ix->gp_radii;
     P.child_counts = ix->child_counts; P.gp_counts = ix->gp_counts; P.used = ix->used;
@@ -779,6 +789,7 @@ static int search_impl(const hira_index_t* ix, const float* q, const float* tau,
     P.flags = flags;
     P.bf_magic = (uint32_t)((0x100000000ull + (uint64_t)bf - 1) / (uint64_t)bf);
     P.ring_offset = 0;
+    P.chained = 0;
     P.ng = (tile_parents + bf - 1) / bf;
     if (tile_parents % bf == 0) {
         P.tile_gp_shift = -1;
@@ -794,13 +805,52 @@ static int search_impl(const hira_index_t* ix, const float* q, const float* tau,
                            "hira_search: cap_parents=%d too large for tile_parents=%d with bf=%d", ix->cap_parents, tile_parents, bf);
         }
     }
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    // int8 pre-filter on the tensor cores when the index carries the side copy and the call allows it
-    if (search_q8_applicable(ix, P)) return launch_search_q8(P, ix, max_group, s);
+    return HIRA_OK;
+}
+
+// the streaming kernel, where the int8 pre-filter does not apply
+static int launch_streaming(const SearchParams& P, const hira_index_t* ix, int32_t max_group, cudaStream_t s) {
     const bool wide = ix->dim > 128;
     if (ix->dtype == HIRA_BF16)
         return wide ? dispatch_gt<__nv_bfloat16, 4>(P, max_group, s) : dispatch_gt<__nv_bfloat16, 2>(P, max_group, s);
     return wide ? dispatch_gt<float, 4>(P, max_group, s) : dispatch_gt<float, 2>(P, max_group, s);
+}
+
+static int search_impl(const hira_index_t* ix, const float* q, const float* tau,
+                       const float* scaling, const float* qnorm, const int32_t* q2kv,
+                       int32_t n_qheads, int32_t max_group, int32_t flags,
+                       int32_t tile_parents, float* out_dense, int32_t* out_idx,
+                       float* out_score, int32_t* out_count, uint32_t* stats,
+                       const void* scan_key, int64_t scan_key_stride, unsigned long long* scan_out, void* stream) {
+    SearchParams P;
+    int rc = search_setup(ix, q, tau, scaling, qnorm, q2kv, n_qheads, max_group, flags, tile_parents, out_dense, out_idx,
+                          out_score, out_count, stats, scan_key, scan_key_stride, scan_out, P);
+    if (rc != HIRA_OK) return rc;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    // int8 pre-filter on the tensor cores when the index carries the side copy and the call allows it
+    if (!search_q8_applicable(ix, P)) return launch_streaming(P, ix, max_group, s);
+    rc = launch_q8_prepare(P, ix, max_group, nullptr, s);
+    return rc != HIRA_OK ? rc : launch_search_q8(P, ix, max_group, s);
+}
+
+int hira::query_and_search(const hira_index_t* ix, const RawQuery& raw, const TauFinder* finder, const float* tau,
+                           const int32_t* q2kv, int n_qheads, int max_group, int flags, int tile_parents, int32_t* idx,
+                           float* score, int32_t* count, const void* scan_key, long long scan_key_stride,
+                           unsigned long long* scan_out, cudaStream_t stream) {
+    SearchParams P;
+    int32_t group = max_group;
+    int rc = search_setup(ix, raw.q_hat, finder ? finder->tau : tau, raw.logit_scale, nullptr, q2kv, n_qheads, group, flags,
+                          tile_parents, nullptr, idx, score, count, nullptr, scan_key, scan_key_stride, scan_out, P);
+    if (rc != HIRA_OK) return rc;
+    const bool q8 = search_q8_applicable(ix, P);
+    P.chained = 1;
+    rc = q8 ? launch_q8_prepare(P, ix, group, &raw, stream)
+            : hira_prepare_query(raw.q, raw.dtype, n_qheads, ix->dim, raw.sm_scale, raw.q_hat, raw.logit_scale, stream);
+    if (rc == HIRA_OK && finder)
+        rc = hira_threshold(finder->samples, ix->dtype, ix->n_heads, finder->n_samples, ix->dim, finder->head_stride,
+                            raw.q_hat, q2kv, n_qheads, finder->method, finder->k, finder->tau, stream);
+    if (rc != HIRA_OK) return rc;
+    return q8 ? launch_search_q8(P, ix, group, stream) : launch_streaming(P, ix, group, stream);
 }
 
 extern "C" int hira_search(const hira_index_t* ix, const float* q, const float* tau,

@@ -47,6 +47,7 @@ struct SearchParams {
     unsigned long long* scan_out;      // [n_heads] packed (order_key(score) << 32 | parent slot), atomicMin
     int n_heads, n_qheads, group, depth, bf, dim;
     int cap_parents, cap_gp, tile_parents, n_tiles, n_chunks, flags;
+    int chained;              // q, tau and scaling come from kernels of the same call that may still run: wait for them (grid_wait)
     int n_tiles_active;       // tiles launched (<= n_tiles, which stays the stride of out_count)
     uint32_t ring_offset;     // byte offset of the per-thread prefetch ring in dynamic shared memory
     int ng;                   // grandparents touched by one tile
@@ -130,9 +131,28 @@ __device__ __forceinline__ void load_row_raw(RawChunk<T> (&raw)[NCH], const T* r
 }
 
 
+// A raw query and where its prepared form goes (see hira_prepare_query).
+struct RawQuery {
+    const void* q;
+    int dtype;
+    float sm_scale;
+    float* q_hat;
+    float* logit_scale;
+};
+
 // set by search.cu's host code, consumed by the kernel launchers of both files
+bool search_q8_applicable(const hira_index_t* ix, const SearchParams& P);
+// query terms of the int8 pre-filter out of prepared queries (raw == NULL) or out of raw ones, which it then prepares too
+int launch_q8_prepare(const SearchParams& P, const hira_index_t* ix, int max_group, const RawQuery* raw, cudaStream_t stream);
 int launch_search_q8(const SearchParams& P, const hira_index_t* ix, int max_group, cudaStream_t stream);
 int q8_refresh(const hira_index_t* ix, cudaStream_t s, long long parents_bound);
-bool search_q8_applicable(const hira_index_t* ix, const SearchParams& P);
+
+// One decode step's query preparation, optional threshold (samples != NULL: found into tau_scratch) and
+// search, as a chain of programmatic launches.  Arguments as in hira_prepare_query, hira_threshold and hira_search.
+struct TauFinder { const void* samples; int n_samples; long long head_stride; int method, k; float* tau; };
+int query_and_search(const hira_index_t* ix, const RawQuery& raw, const TauFinder* finder, const float* tau,
+                     const int32_t* q2kv, int n_qheads, int max_group, int flags, int tile_parents, int32_t* idx,
+                     float* score, int32_t* count, const void* scan_key, long long scan_key_stride,
+                     unsigned long long* scan_out, cudaStream_t stream);
 
 }  // namespace hira

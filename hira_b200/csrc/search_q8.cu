@@ -130,15 +130,20 @@ __device__ __forceinline__ void worker_reduce(float (&v)[GT], float (*s_red)[8],
 // channel t.  q' = q (.) s is split into two int8 terms, q' = c1 a1 + c2 a2 + r2; out = 16 rows of
 // 128 int8 (row 2j = a1 of head j, row 2j+1 = a2; 16-byte chunks swizzled by the row; absent heads
 // zero) followed by (c1, c2, A, B) per head with A >= ||q'||_2, B >= 127 ||r2||_1 + rounding.
+// RAW: q holds the caller's queries; they are normalised here first (the arithmetic of
+// prepare_query_kernel, one channel per thread) and written to q_hat / logit_scale, which saves the decode
+// step a launch.
+template <typename TQ, bool RAW>
 __global__ void __launch_bounds__(Q8_WORKERS)
-search_q8_prepare_kernel(const float* __restrict__ q, const float* __restrict__ chan_scale, float* chan_scale_rw,
-                         int group, int gt, int dim, unsigned char* __restrict__ out) {
+search_q8_prepare_kernel(const TQ* __restrict__ q, const float* __restrict__ chan_scale, float* chan_scale_rw,
+                         int group, int gt, int dim, unsigned char* __restrict__ out, float sm_scale,
+                         float* __restrict__ q_hat, float* __restrict__ logit_scale) {
     constexpr int GT = 4;
     __shared__ float s_red[4][8];
     // The search kernel behind this one is launched with programmatic stream serialisation: its CTAs may
     // start (barriers, tensor memory, gates) while this grid runs, and wait for it (griddepcontrol.wait)
     // where they first need the query terms or the hint words.
-    asm volatile("griddepcontrol.launch_dependents;");
+    grid_trigger();
     const int tid = threadIdx.x, warp = tid >> 5, wl = tid & 31;
     const int chunk = blockIdx.x, h = blockIdx.y;
     int nq = group - chunk * gt;
@@ -146,8 +151,30 @@ search_q8_prepare_kernel(const float* __restrict__ q, const float* __restrict__ 
     const float cs = chan_scale[(size_t)h * HIRA_Q8_CHAN + tid];
     float qp[GT], v[GT];
 #pragma unroll
+    for (int j = 0; j < GT; ++j) qp[j] = j < nq ? (float)q[(size_t)(h * group + chunk * gt + j) * dim + tid] : 0.f;
+    if (RAW) {
+#pragma unroll
+        for (int j = 0; j < GT; ++j) {
+            v[j] = __fmaf_rn(qp[j], qp[j], 0.f);
+#pragma unroll
+            for (int s = 16; s >= 1; s >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], s);
+            if (wl == 0) s_red[warp][j] = v[j];
+        }
+        worker_sync();
+#pragma unroll
+        for (int j = 0; j < GT; ++j) {
+            const float nrm = fmaxf(__fsqrt_rn(s_red[0][j] + s_red[1][j] + s_red[2][j] + s_red[3][j]), 1e-20f);
+            qp[j] = __fdiv_rn(qp[j], nrm);
+            if (j < nq) {
+                const size_t qh = (size_t)h * group + chunk * gt + j;
+                q_hat[qh * dim + tid] = qp[j];
+                if (tid == 0) logit_scale[qh] = nrm * sm_scale;
+            }
+        }
+    }
+#pragma unroll
     for (int j = 0; j < GT; ++j) {
-        qp[j] = j < nq ? q[(size_t)(h * group + chunk * gt + j) * dim + tid] * cs : 0.f;
+        qp[j] *= cs;
         v[j] = fabsf(qp[j]);
     }
     worker_reduce<GT, true>(v, s_red, warp, wl);
@@ -378,7 +405,7 @@ search_q8_kernel(const SearchParams P, const int8_t* __restrict__ k8, const uint
             for (int i = 0; i < spec; ++i) order[i] = i;
             for (; issued < spec && issued < Q8_SLOTS; ++issued) issue(issued);
             Q8_STAMP(8, Q8_WORKERS);
-            asm volatile("griddepcontrol.wait;" ::: "memory");   // the query terms are written
+            grid_wait();   // the query terms are written
             mbar_expect_tx(bar_q, Q8_QBYTES);
             bulk_load(s_base + Q8Smem::BQ, qterms + ((size_t)h * P.n_chunks + chunk) * Q8_QBYTES, Q8_QBYTES, bar_q);
             for (int k = 0; !failed; ++k) {
@@ -427,28 +454,6 @@ search_q8_kernel(const SearchParams P, const int8_t* __restrict__ k8, const uint
         const int g0 = P.tile_gp_shift >= 0 ? (tile >> P.tile_gp_shift)
                                             : (P.tile_gp_shift == -1 ? tile * P.ng : div_bf(tile * TP, bf, P.bf_magic));
         const int ng = P.ng;
-        int my_qh = qh_of[0];
-#pragma unroll
-        for (int j = 1; j < GT; ++j)
-            if (my_head == j) my_qh = qh_of[j];
-        const float my_tau = head_on ? P.tau[my_qh] : 0.f;
-        const float my_qn = 1.f;
-        if (tid < nq) {
-            s_scale[tid] = P.scaling ? P.scaling[s_qh[tid]] : 1.0f;
-            s_tau[tid] = P.tau[s_qh[tid]];
-        }
-        float qreg[GT][NCH][8];
-#pragma unroll
-        for (int j = 0; j < GT; ++j) {
-            if (j < nq) {
-                load_vec_f32<NCH>(P.q + (size_t)qh_of[j] * P.dim, qreg[j], lane, P.dim);
-            } else {
-#pragma unroll
-                for (int i = 0; i < NCH; ++i)
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) qreg[j][i][e] = 0.f;
-            }
-        }
         // gate inputs, issued together (as in search.cu)
         RawChunk<T> graw[NCH];
         float grad = 0.f;
@@ -470,6 +475,29 @@ search_q8_kernel(const SearchParams P, const int8_t* __restrict__ k8, const uint
             prad[u] = in ? P.parent_radii[(size_t)h * P.cap_parents + p] : 0.f;
             pcnt[u] = in ? P.child_counts[(size_t)h * P.cap_parents + p] : 0;
             pgc[u] = (in && P.depth == 3) ? P.gp_counts[(size_t)h * P.cap_gp + g0 + div_bf(p - g0 * bf, bf, P.bf_magic)] : 0;
+        }
+        if (P.chained) grid_wait();   // the query, its threshold and scale come from the kernels just before
+        int my_qh = qh_of[0];
+#pragma unroll
+        for (int j = 1; j < GT; ++j)
+            if (my_head == j) my_qh = qh_of[j];
+        const float my_tau = head_on ? P.tau[my_qh] : 0.f;
+        const float my_qn = 1.f;
+        if (tid < nq) {
+            s_scale[tid] = P.scaling ? P.scaling[s_qh[tid]] : 1.0f;
+            s_tau[tid] = P.tau[s_qh[tid]];
+        }
+        float qreg[GT][NCH][8];
+#pragma unroll
+        for (int j = 0; j < GT; ++j) {
+            if (j < nq) {
+                load_vec_f32<NCH>(P.q + (size_t)qh_of[j] * P.dim, qreg[j], lane, P.dim);
+            } else {
+#pragma unroll
+                for (int i = 0; i < NCH; ++i)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) qreg[j][i][e] = 0.f;
+            }
         }
         const bool do_scan = SCAN && chunk == 0;
         float psq[PRE];
@@ -642,7 +670,7 @@ search_q8_kernel(const SearchParams P, const int8_t* __restrict__ k8, const uint
         if (tid == 0) {
             mbar_arrive(bar_go);
             if (chunk == 0 && tile_in_use) {   // what the gates kept, for the next search's streaming mode
-                asm volatile("griddepcontrol.wait;" ::: "memory");   // the counters of the last search are consumed
+                grid_wait();   // the counters of the last search are consumed
                 atomicAdd(hint, (uint32_t)__popc(*reinterpret_cast<volatile int*>(&s_need)));
                 atomicAdd(hint + 1, (uint32_t)n_stage_tile);
             }
@@ -844,24 +872,12 @@ static int launch_q8(SearchParams P, int chunks, const hira_index_t* ix, cudaStr
     P.n_chunks = chunks;
     HIRA_CHECK_ARG(P.n_tiles <= 65535 && P.n_heads <= 65535, HIRA_ERR_SHAPE,
                    "hira_search: %d tiles x %d heads exceed the grid limits", P.n_tiles, P.n_heads);
-    unsigned char* qterms = reinterpret_cast<unsigned char*>(ix->q8_query_scratch);
-    search_q8_prepare_kernel<<<dim3((unsigned)chunks, (unsigned)P.n_heads), Q8_WORKERS, 0, stream>>>(
-        P.q, ix->q8_chan_scale, ix->q8_chan_scale, P.group, GT, P.dim, qterms);
-    HIRA_CHECK_LAUNCH("hira_search (int8 pre-filter, query terms) launch");
     // launched so that its CTAs may start while the query terms are still being prepared (see above)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)chunks, (unsigned)P.n_tiles_active, (unsigned)P.n_heads);
-    cfg.blockDim = dim3(Q8_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, P, reinterpret_cast<const int8_t*>(ix->children_q8),
-                           reinterpret_cast<const uint32_t*>(ix->children_q8_meta),
-                           reinterpret_cast<const unsigned char*>(qterms), reinterpret_cast<uint32_t*>(ix->q8_chan_scale));
+    e = launch_chained(kern, dim3((unsigned)chunks, (unsigned)P.n_tiles_active, (unsigned)P.n_heads), dim3(Q8_THREADS), smem,
+                       stream, P, reinterpret_cast<const int8_t*>(ix->children_q8),
+                       reinterpret_cast<const uint32_t*>(ix->children_q8_meta),
+                       reinterpret_cast<const unsigned char*>(ix->q8_query_scratch),
+                       reinterpret_cast<uint32_t*>(ix->q8_chan_scale));
     if (e != cudaSuccess) {
         set_error("hira_search (int8 pre-filter) launch: %s", cudaGetErrorString(e));
         return HIRA_ERR_CUDA;
@@ -886,9 +902,36 @@ bool search_q8_applicable(const hira_index_t* ix, const SearchParams& P) {
     return true;
 }
 
-int launch_search_q8(const SearchParams& P, const hira_index_t* ix, int max_group, cudaStream_t stream) {
+static int q8_heads_per_chunk(int max_group) {
     int gt = 1;
     while (gt < max_group && gt < 4) gt <<= 1;
+    return gt;
+}
+
+int launch_q8_prepare(const SearchParams& P, const hira_index_t* ix, int max_group, const RawQuery* raw, cudaStream_t stream) {
+    const int gt = q8_heads_per_chunk(max_group);
+    const dim3 grid((unsigned)((max_group + gt - 1) / gt), (unsigned)P.n_heads);
+    unsigned char* qterms = reinterpret_cast<unsigned char*>(ix->q8_query_scratch);
+    if (raw == nullptr) {
+        search_q8_prepare_kernel<float, false><<<grid, Q8_WORKERS, 0, stream>>>(
+            P.q, ix->q8_chan_scale, ix->q8_chan_scale, P.group, gt, P.dim, qterms, 0.f, nullptr, nullptr);
+    } else {
+        HIRA_CHECK_ARG(raw->dtype == HIRA_F32 || raw->dtype == HIRA_BF16, HIRA_ERR_DTYPE, "hira_prepare_query: dtype %d", raw->dtype);
+        if (raw->dtype == HIRA_BF16)
+            search_q8_prepare_kernel<__nv_bfloat16, true><<<grid, Q8_WORKERS, 0, stream>>>(
+                reinterpret_cast<const __nv_bfloat16*>(raw->q), ix->q8_chan_scale, ix->q8_chan_scale, P.group, gt, P.dim,
+                qterms, raw->sm_scale, raw->q_hat, raw->logit_scale);
+        else
+            search_q8_prepare_kernel<float, true><<<grid, Q8_WORKERS, 0, stream>>>(
+                reinterpret_cast<const float*>(raw->q), ix->q8_chan_scale, ix->q8_chan_scale, P.group, gt, P.dim, qterms,
+                raw->sm_scale, raw->q_hat, raw->logit_scale);
+    }
+    HIRA_CHECK_LAUNCH("hira_search (int8 pre-filter, query terms) launch");
+    return HIRA_OK;
+}
+
+int launch_search_q8(const SearchParams& P, const hira_index_t* ix, int max_group, cudaStream_t stream) {
+    const int gt = q8_heads_per_chunk(max_group);
     const int chunks = (max_group + gt - 1) / gt;
     const bool bf16 = ix->dtype == HIRA_BF16;
     switch (gt) {

@@ -58,6 +58,8 @@ threshold_kernel(const T* __restrict__ samples, long long head_stride, int n_sam
     constexpr int ROWS = 16 / ((int)sizeof(T) * NCH);   // 128 bytes of rows in flight per lane
     __shared__ uint32_t s[TAU_MAX_SAMPLES];
     const int tid = threadIdx.x, lane = tid & (GROUP - 1), hw = tid / GROUP, warp = tid >> 5, wl = tid & 31;
+    grid_wait();
+    grid_trigger();
     const int qh = blockIdx.x;
     const int h = q2kv ? q2kv[qh] : qh / group;
     const T* rows = samples + (size_t)h * head_stride;
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(128)
 prepare_query_kernel(const T* __restrict__ q, int dim, float sm_scale, float* __restrict__ q_hat,
                      float* __restrict__ logit_scale) {
     __shared__ float s_part[4];
+    grid_trigger();   // launched plainly: everything before it is complete
     const int qh = blockIdx.x, tid = threadIdx.x;
     const T* row = q + (size_t)qh * dim;
     float acc = 0.f;
@@ -249,16 +252,21 @@ extern "C" int hira_threshold(const void* samples, int32_t dtype, int32_t n_head
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int group = q2kv ? 1 : n_qheads / n_heads;
     const bool wide = dim > 128;  // chunks per lane: 2 up to 128 elements, else 4
+    const dim3 grid((unsigned)n_qheads);
+    cudaError_t e;
     if (dtype == HIRA_BF16) {
         auto* p = reinterpret_cast<const __nv_bfloat16*>(samples);
-        if (wide) threshold_kernel<__nv_bfloat16, 4, 512><<<n_qheads, 512, 0, s>>>(p, head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
-        else threshold_kernel<__nv_bfloat16, 2, 1024><<<n_qheads, 1024, 0, s>>>(p, head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
+        if (wide) e = launch_chained(threshold_kernel<__nv_bfloat16, 4, 512>, grid, dim3(512), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
+        else e = launch_chained(threshold_kernel<__nv_bfloat16, 2, 1024>, grid, dim3(1024), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
     } else {
         auto* p = reinterpret_cast<const float*>(samples);
-        if (wide) threshold_kernel<float, 4, 512><<<n_qheads, 512, 0, s>>>(p, head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
-        else threshold_kernel<float, 2, 1024><<<n_qheads, 1024, 0, s>>>(p, head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
+        if (wide) e = launch_chained(threshold_kernel<float, 4, 512>, grid, dim3(512), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
+        else e = launch_chained(threshold_kernel<float, 2, 1024>, grid, dim3(1024), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
     }
-    HIRA_CHECK_LAUNCH("hira_threshold launch");
+    if (e != cudaSuccess) {
+        set_error("hira_threshold launch: %s", cudaGetErrorString(e));
+        return HIRA_ERR_CUDA;
+    }
     return HIRA_OK;
 }
 

@@ -388,9 +388,11 @@ def prepare_query(q: torch.Tensor, sm_scale: float, q_hat=None, logit_scale=None
 def decode_attention(st: IndexState, q: torch.Tensor, sm_scale: float, tau: torch.Tensor, compact: CompactResult,
                      q_hat: torch.Tensor, logit_scale: torch.Tensor, *, q2kv=None, max_group: int = 0, flags: int = 0,
                      queued_k=None, queued_v=None, n_splits: int, workspace: torch.Tensor, out: torch.Tensor,
-                     out_ml=None, scan_key=None, scan_out=None, searched_event=None):
+                     out_ml=None, scan_key=None, scan_out=None, searched_event=None, tau_samples=None,
+                     tau_method: int = 0, tau_k: int = 1):
     """prepare_query + search (compact) + sparse_attn in one library call.  q (H_q, D) fp32/bf16
-    contiguous; everything else preallocated by the caller."""
+    contiguous; everything else preallocated by the caller.  With `tau_samples` (H_kv, S, D) in the index
+    dtype the threshold is found on the way, into `tau`."""
     lib = L.load()
     hq = q.shape[0]
     n_queued, qstride = 0, 0
@@ -401,15 +403,21 @@ def decode_attention(st: IndexState, q: torch.Tensor, sm_scale: float, tau: torc
         qstride = n_queued * st.dim
         if st.vdim != st.dim:
             raise ValueError("queued keys/values with vdim != dim are not supported")
-    rc = lib.hira_decode_attention(st.struct, L.ptr(q), L.dtype_code(q.dtype), float(sm_scale), L.ptr(tau), L.ptr(q2kv),
-                                   hq, max_group, flags, compact.tile_parents, L.ptr(q_hat), L.ptr(logit_scale),
-                                   L.ptr(compact.idx), L.ptr(compact.score), L.ptr(compact.count),
-                                   L.ptr(queued_k) if n_queued else None, L.ptr(queued_v) if n_queued else None,
-                                   n_queued, qstride, n_splits, L.ptr(workspace), L.ptr(out), L.ptr(out_ml),
-                                   out.stride(0), out_ml.stride(0) if out_ml is not None else 0,
-                                   L.ptr(scan_key) if scan_out is not None else None,
-                                   scan_key.stride(0) if scan_out is not None else 0, L.ptr(scan_out),
-                                   searched_event, L.current_stream(st.device))
+    rest = (L.ptr(q2kv), hq, max_group, flags, compact.tile_parents, L.ptr(q_hat), L.ptr(logit_scale),
+            L.ptr(compact.idx), L.ptr(compact.score), L.ptr(compact.count),
+            L.ptr(queued_k) if n_queued else None, L.ptr(queued_v) if n_queued else None,
+            n_queued, qstride, n_splits, L.ptr(workspace), L.ptr(out), L.ptr(out_ml),
+            out.stride(0), out_ml.stride(0) if out_ml is not None else 0,
+            L.ptr(scan_key) if scan_out is not None else None,
+            scan_key.stride(0) if scan_out is not None else 0, L.ptr(scan_out),
+            searched_event, L.current_stream(st.device))
+    if tau_samples is None:
+        rc = lib.hira_decode_attention(st.struct, L.ptr(q), L.dtype_code(q.dtype), float(sm_scale), L.ptr(tau), *rest)
+    else:
+        assert tau_samples.dtype == st.dtype and tau_samples.is_contiguous() and tau_samples.shape[0] == st.n_heads
+        rc = lib.hira_decode_attention_sampled(st.struct, L.ptr(q), L.dtype_code(q.dtype), float(sm_scale),
+                                               L.ptr(tau_samples), tau_samples.shape[1], tau_samples.stride(0),
+                                               tau_method, tau_k, L.ptr(tau), *rest)
     L.check(rc, "hira_decode_attention")
     compact.n_tiles_active = None if st.active_parents == 0 else -(-st.active_parents // compact.tile_parents)
     return out

@@ -361,6 +361,20 @@ int hira_decode_attention(const hira_index_t* index, const void* q, int32_t q_dt
                           const void* scan_key, int64_t scan_key_stride, uint64_t* scan_out,
                           void* searched, void* stream);
 
+/* The same with the threshold found on the way (hira_threshold on `tau_samples` in the index dtype, one
+ * set of `n_samples` rows per kv head, heads `samples_head_stride` elements apart) and left in tau [n_qheads]. */
+int hira_decode_attention_sampled(const hira_index_t* index, const void* q, int32_t q_dtype, float sm_scale,
+                                  const void* tau_samples, int32_t n_samples, int64_t samples_head_stride,
+                                  int32_t tau_method, int32_t tau_k, float* tau,
+                                  const int32_t* q2kv, int32_t n_qheads, int32_t max_group,
+                                  int32_t flags, int32_t tile_parents, float* q_hat, float* logit_scale,
+                                  int32_t* idx, float* score, int32_t* count,
+                                  const void* queued_k, const void* queued_v, int32_t n_queued,
+                                  int64_t queued_head_stride, int32_t n_splits, float* workspace,
+                                  float* out, float* out_ml, int64_t out_head_stride, int64_t ml_head_stride,
+                                  const void* scan_key, int64_t scan_key_stride, uint64_t* scan_out,
+                                  void* searched, void* stream);
+
 /* One whole decode step of one layer from HOST buffers, in one call: the copy of the query to the
  * device, query preparation, the threshold (given, or found on the device from the step's
  * samples), search, sparse attention, the copy of the output back to the host and -- when k_host

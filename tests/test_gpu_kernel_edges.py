@@ -86,3 +86,33 @@ def test_merge_partials_edges(n_parts, vdim, hq):
     # weights by __expf (2 ulp + 2^-21 |x|, |x| <= 40) and fp32 sums of n_parts terms
     assert (got - want).norm() / want.norm() < 4e-6 + n_parts * 6e-8
     assert torch.equal(out_ml[:, 0].cpu(), ml[..., 0].max(dim=0).values)
+
+
+@pytest.mark.parametrize("d,group,qdtype,dtype", [(128, 1, torch.float32, torch.float32), (128, 3, torch.bfloat16, torch.bfloat16),
+                                                  (128, 5, torch.bfloat16, torch.bfloat16), (128, 16, torch.float32, torch.bfloat16),
+                                                  (128, 17, torch.bfloat16, torch.bfloat16), (64, 4, torch.bfloat16, torch.bfloat16),
+                                                  (200, 2, torch.float32, torch.float32)])
+def test_sampled_decode_entry_equals_the_separate_calls(d, group, qdtype, dtype):
+    """Query preparation (inside the pre-filter's own or on its own), threshold, search and attention as one chain
+    of launches, again and again on one stream, against the same calls one by one."""
+    h, bf, n = 3, 32, 3000
+    st, _, keys, _ = build_both(h, n, d, bf, 3, dtype, seed=71, spare=bf)
+    st.refresh_int8_copy()
+    hq = h * group
+    flags = L.HIRA_GATE_GE | L.HIRA_LEAF_GE
+    samples = keys[:, ::7].contiguous()
+    compact = S.alloc_compact(st, hq)
+    n_splits = S.attn_splits(st, hq)
+    f32 = dict(dtype=torch.float32, device="cuda")
+    ws = torch.empty((hq * n_splits * (d + 2),), **f32)
+    q_hat, scale, tau = torch.empty((hq, d), **f32), torch.empty((hq,), **f32), torch.empty((hq,), **f32)
+    for step in range(4):
+        q = (make_queries(hq, d, seed=80 + step, normalize=False) * 3).to(qdtype)
+        out = S.decode_attention(st, q, 0.1, tau, compact, q_hat, scale, flags=flags, n_splits=n_splits, workspace=ws,
+                                 out=torch.empty((hq, d), **f32), tau_samples=samples, tau_method=L.HIRA_TAU_SAMPLE_MEAN_TOPK, tau_k=9)
+        want_q, want_s = S.prepare_query(q, 0.1)
+        want_tau = S.threshold(samples, want_q, L.HIRA_TAU_SAMPLE_MEAN_TOPK, 9)
+        _, c2 = S.search(st, want_q, want_tau, scaling=want_s, flags=flags, want_compact=True)
+        want = S.sparse_attn(st, want_q, want_s, c2, n_splits=n_splits)
+        for a, b in ((q_hat, want_q), (scale, want_s), (tau, want_tau), (compact.count, c2.count), (out, want)):
+            assert torch.equal(a, b)
