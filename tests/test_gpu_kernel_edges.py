@@ -116,3 +116,13 @@ def test_sampled_decode_entry_equals_the_separate_calls(d, group, qdtype, dtype)
         want = S.sparse_attn(st, want_q, want_s, c2, n_splits=n_splits)
         for a, b in ((q_hat, want_q), (scale, want_s), (tau, want_tau), (compact.count, c2.count), (out, want)):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_export_to_unaligned_outputs(dtype):
+    st, _, keys, vals = build_both(2, 300, 40, 8, 3, dtype, seed=9)
+    e = torch.finfo(dtype).bits // 8
+    out_k, out_v = (torch.zeros(2 * 300 * 40 * e + 16, dtype=torch.uint8, device="cuda")[e:] for _ in range(2))
+    L.check(L.load().hira_export(st.struct, 0, 300, out_k.data_ptr(), out_v.data_ptr(), L.current_stream()))
+    for out, want in ((out_k, keys), (out_v, vals)):
+        assert torch.equal(out[: want.numel() * e].clone(), want.contiguous().view(torch.uint8).flatten())
