@@ -118,6 +118,16 @@ def test_sampled_decode_entry_equals_the_separate_calls(d, group, qdtype, dtype)
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("dtype,d", [(torch.float32, 8), (torch.float32, 128), (torch.bfloat16, 72), (torch.float32, 256)])
+@pytest.mark.parametrize("n,k", [(1, 1), (127, 63), (128, 64), (129, 65), (300, 200)])
+def test_assign_tile_edges(dtype, d, n, k):
+    pts, cents = make_keys(2, n, d, 7, dtype), make_keys(2, k, d, 8, dtype)
+    cents[:, k // 2:] = cents[:, : k - k // 2]            # equal centres: the lower one wins
+    idx, d2 = S.assign(pts, cents)
+    want_i, want_d = O.assign(pts, cents)
+    assert np.array_equal(idx.cpu().numpy(), want_i) and np.array_equal(d2.cpu().numpy().view(np.uint32), want_d.view(np.uint32))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_export_to_unaligned_outputs(dtype):
     st, _, keys, vals = build_both(2, 300, 40, 8, 3, dtype, seed=9)
