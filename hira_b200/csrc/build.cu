@@ -17,7 +17,7 @@
 // per-head randperm, optional Lloyd mean updates precede the final assignment,
 // and counts/validity are written as explicit state.
 #include "common.cuh"
-#include <cub/cub.cuh>
+#include <cub/block/block_scan.cuh>
 #include <math_constants.h>
 #include <string.h>
 
@@ -273,45 +273,165 @@ __global__ void gather_centres_kernel(const T* __restrict__ points, long long p_
     for (int e = 0; e < 8; ++e) w[e] = r[e];
 }
 
+// ---------------------------------------------------------------------------
+// Members of every centre in (distance, point) order.
+//
+// The points of a head are counted per centre, the counts scanned, the points dropped into their centre's
+// range in arrival order and each range sorted by itself: a range is bf points on average, so nearly all of
+// them are sorted by one warp in registers.  The sort key is (distance bits, point), which no two members
+// share, so the result does not depend on the arrival order.  (A device-wide radix sort of (centre, distance)
+// before: 5 or 6 passes of about 9 us whatever the size; 8 x 32,768 points in
+// 1,024 centres each 65 -> 30 us, 8 x 4,096 points in 64 73 -> 22 us with all of the kernels around it.)
+// ---------------------------------------------------------------------------
+
 // An assignment outside [0, k) -- the tensor-core kernel writes -1 for the points of a CTA whose
 // bounded barrier wait ran out -- must not reach the segment arithmetic below: the point goes to
 // centre 0 at distance 0 (so that every later index stays in range) and the caller is told through
 // the status word.
-// `placed` (balanced rounds): points that already have a slot sort behind every real segment.
-__global__ void make_sort_keys_kernel(const int32_t* __restrict__ idx, const float* __restrict__ d2, int n, int k,
-                                      long long total, long long n_seg, const int32_t* __restrict__ placed,
-                                      uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                      int32_t* __restrict__ status) {
+// `placed` (balanced rounds): points that already have a slot belong to no centre any more (arrival -1).
+__global__ void count_members_kernel(int32_t* __restrict__ idx, float* __restrict__ d2, int n, int k, long long total,
+                                     const int32_t* __restrict__ placed, int32_t* __restrict__ cnt,
+                                     int32_t* __restrict__ arrival, int32_t* __restrict__ status) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
-    const int h = (int)(i / n);
     if (placed && placed[i] >= 0) {
-        keys[i] = (uint64_t)n_seg << 32;
-        vals[i] = (uint32_t)(i - (long long)h * n);
+        arrival[i] = -1;
         return;
     }
     int c = idx[i];
-    float d = d2[i];
-    if (c < 0 || c >= k || !(d >= 0.f)) {
+    if (c < 0 || c >= k || !(d2[i] >= 0.f)) {
         if (status) atomicOr(status, HIRA_STATUS_ASSIGN_FAILED);
-        c = 0;
-        d = 0.f;
+        idx[i] = c = 0;
+        d2[i] = 0.f;
     }
-    const uint64_t seg = (uint64_t)h * k + (uint32_t)c;
-    keys[i] = (seg << 32) | (uint64_t)__float_as_uint(d);  // d >= 0: bits order like values
-    vals[i] = (uint32_t)(i - (long long)h * n);
+    arrival[i] = atomicAdd(cnt + (i / n) * k + c, 1);
 }
 
-// start[s] = first sorted position whose segment id >= s, for s in [0, n_seg]
-__global__ void segment_starts_kernel(const uint64_t* __restrict__ keys, long long total, long long n_seg,
-                                      int32_t* __restrict__ start) {
+// start[h][c] = h n + members of the centres before c
+constexpr int SCAN_ITEMS = 4;
+__global__ void __launch_bounds__(1024)
+member_starts_kernel(const int32_t* __restrict__ cnt, int n, int k, int32_t* __restrict__ start) {
+    typedef cub::BlockScan<int, 1024> Scan;
+    __shared__ typename Scan::TempStorage tmp;
+    const int h = blockIdx.x;
+    int carry = h * n;
+    for (int c0 = 0; c0 < k; c0 += 1024 * SCAN_ITEMS) {
+        int v[SCAN_ITEMS], total;
+        const int c = c0 + threadIdx.x * SCAN_ITEMS;
+#pragma unroll
+        for (int u = 0; u < SCAN_ITEMS; ++u) v[u] = c + u < k ? cnt[(size_t)h * k + c + u] : 0;
+        Scan(tmp).ExclusiveSum(v, v, total);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < SCAN_ITEMS; ++u)
+            if (c + u < k) start[(size_t)h * k + c + u] = carry + v[u];
+        carry += total;
+    }
+}
+
+__global__ void drop_members_kernel(const int32_t* __restrict__ idx, const float* __restrict__ d2, int n, int k,
+                                    long long total, const int32_t* __restrict__ start, const int32_t* __restrict__ arrival,
+                                    uint64_t* __restrict__ keys) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > total) return;
-    long long cur = (i < total) ? (long long)(keys[i] >> 32) : n_seg;
-    long long prev = (i == 0) ? -1 : (long long)(keys[i - 1] >> 32);
-    cur = cur > n_seg ? n_seg : cur;     // `start` has n_seg + 1 entries
-    prev = prev > n_seg ? n_seg : prev;
-    for (long long s = prev + 1; s <= cur; ++s) start[s] = (int32_t)i;
+    if (i >= total) return;
+    const int a = arrival[i];
+    if (a < 0) return;
+    const long long h = i / n;
+    // d2 >= 0: bits order like values
+    keys[start[h * k + idx[i]] + a] = ((uint64_t)__float_as_uint(d2[i]) << 32) | (uint32_t)(i - h * n);
+}
+
+// Eight ranges per CTA.  Up to SORT_WARP members: one warp, the rank of a member is the number of smaller keys.
+// Up to SORT_CTA: the CTA sorts the range in shared memory (bitonic).  Longer ones (many equal points): sorted
+// pieces of SORT_CTA, then merged pairwise through the second key array, each member finding its place in the
+// sibling piece by bisection.  Writes the member list and the rank of every point inside its range.
+constexpr int SORT_THREADS = 256, SORT_RANGES = SORT_THREADS / 32, SORT_WARP = 128, SORT_CTA = 4096;
+__global__ void __launch_bounds__(SORT_THREADS)
+sort_members_kernel(const int32_t* __restrict__ cnt, const int32_t* __restrict__ start, int n, int k, long long n_seg,
+                    uint64_t* __restrict__ keys, uint64_t* __restrict__ keys2, uint32_t* __restrict__ sorted_ids,
+                    int32_t* __restrict__ rank) {
+    __shared__ uint64_t sk[SORT_CTA];   // SORT_RANGES x SORT_WARP of it while the warps work
+    const int tid = threadIdx.x, warp = tid >> 5, wl = tid & 31;
+    const long long seg0 = (long long)blockIdx.x * SORT_RANGES;
+    {
+        const long long seg = seg0 + warp;
+        const int m = seg < n_seg ? cnt[seg] : 0;
+        if (m > 0 && m <= SORT_WARP) {
+            const int b = start[seg];
+            const size_t head = (size_t)(seg / k) * n;
+            uint64_t* mine = sk + warp * SORT_WARP;
+            for (int i = wl; i < m; i += 32) mine[i] = keys[b + i];
+            __syncwarp();
+            for (int i = wl; i < m; i += 32) {
+                const uint64_t key = mine[i];
+                int r = 0;
+                for (int j = 0; j < m; ++j) r += mine[j] < key ? 1 : 0;
+                const uint32_t id = (uint32_t)key;
+                sorted_ids[b + r] = id;
+                rank[head + id] = r;
+            }
+        }
+    }
+    for (int w = 0; w < SORT_RANGES; ++w) {   // every test below is uniform over the CTA
+        const long long seg = seg0 + w;
+        const int m = seg < n_seg ? cnt[seg] : 0;
+        if (m <= SORT_WARP) continue;
+        const int b = start[seg];
+        const size_t head = (size_t)(seg / k) * n;
+        uint64_t *from = keys + b, *to = keys2 + b;
+        for (int p0 = 0; p0 < m; p0 += SORT_CTA) {
+            const int np = min(m - p0, SORT_CTA);
+            int n2 = 2 * SORT_WARP;
+            while (n2 < np) n2 <<= 1;
+            __syncthreads();
+            for (int i = tid; i < n2; i += SORT_THREADS) sk[i] = i < np ? from[p0 + i] : ~0ull;
+            __syncthreads();
+            for (int size = 2; size <= n2; size <<= 1) {
+                for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                    for (int t = tid; t < n2 / 2; t += SORT_THREADS) {
+                        const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+                        const bool up = (i & size) == 0;
+                        const uint64_t x = sk[i], y = sk[j];
+                        if ((x > y) == up) { sk[i] = y; sk[j] = x; }
+                    }
+                    __syncthreads();
+                }
+            }
+            if (m <= SORT_CTA) {
+                for (int i = tid; i < np; i += SORT_THREADS) {
+                    const uint32_t id = (uint32_t)sk[i];
+                    sorted_ids[b + i] = id;
+                    rank[head + id] = i;
+                }
+            } else {
+                for (int i = tid; i < np; i += SORT_THREADS) from[p0 + i] = sk[i];
+            }
+        }
+        if (m <= SORT_CTA) continue;
+        for (int len = SORT_CTA; len < m; len *= 2) {
+            __syncthreads();   // the pieces written above (or in the pass before) are visible to the whole CTA
+            const bool last = 2 * (long long)len >= m;
+            for (int i = tid; i < m; i += SORT_THREADS) {
+                const int piece = i / len, sib = piece ^ 1;
+                int lo = min(sib * len, m), hi = min(lo + len, m);
+                const int sib0 = lo;
+                const uint64_t key = from[i];
+                while (lo < hi) {   // members of the sibling piece that come before this one
+                    const int mid = (lo + hi) >> 1;
+                    if (from[mid] < key) lo = mid + 1; else hi = mid;
+                }
+                const int at = (piece & ~1) * len + (i - piece * len) + (lo - sib0);
+                if (last) {
+                    const uint32_t id = (uint32_t)key;
+                    sorted_ids[b + at] = id;
+                    rank[head + id] = at;
+                } else {
+                    to[at] = key;
+                }
+            }
+            uint64_t* t = from; from = to; to = t;
+        }
+    }
 }
 
 // Lloyd mean update.  The members of a centre are added one after another in sorted order, so a centre is
@@ -341,7 +461,8 @@ template <> struct MeansElem<__nv_bfloat16> {
 template <typename T>
 __global__ void __launch_bounds__(256)
 means_kernel(const T* __restrict__ points, long long p_head_stride, int n, const uint32_t* __restrict__ sorted_ids,
-             const int32_t* __restrict__ start, int k, int dim, int slabs, long long n_seg, T* __restrict__ cents) {
+             const int32_t* __restrict__ start, const int32_t* __restrict__ count, int k, int dim, int slabs,
+             long long n_seg, T* __restrict__ cents) {
     typedef MeansElem<T> E;
     typedef typename E::raw raw_t;
     const int wl = threadIdx.x & 31;
@@ -350,7 +471,7 @@ means_kernel(const T* __restrict__ points, long long p_head_stride, int n, const
     if (seg >= n_seg) return;   // the whole warp
     const int d = ((int)(w - seg * slabs) * 32 + wl) * E::N;
     const int h = (int)(seg / k);
-    const int b = start[seg], e = start[seg + 1];
+    const int b = start[seg], e = b + count[seg];
     if (e <= b) return;  // empty cluster keeps its centre
     const bool on = d < dim;
     const T* P = points + (size_t)h * p_head_stride + (on ? d : 0);
@@ -394,37 +515,33 @@ __global__ void mask_full_centres_kernel(const float* __restrict__ csq, const in
 
 // An intermediate balanced round: every centre accepts, closest first, as many of the points that
 // chose it as it still has room for; the rest stay unplaced for the next round.
-__global__ void accept_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ sorted_ids,
-                              const int32_t* __restrict__ start, const int32_t* __restrict__ filled, int n, int k,
-                              int bf, long long total, long long n_seg, int32_t* __restrict__ slot) {
-    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= total) return;
-    const long long seg = (long long)(keys[j] >> 32);
-    if (seg >= n_seg) return;   // placed earlier
-    const int h = (int)(seg / k);
-    const int c = (int)(seg - (long long)h * k);
-    const int rank = (int)(j - start[seg]);
-    const int have = filled[seg];
-    if (rank < bf - have) slot[(size_t)h * n + sorted_ids[j]] = c * bf + have + rank;
+__global__ void accept_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ rank,
+                              const int32_t* __restrict__ filled, int n, int k, int bf, long long total,
+                              int32_t* __restrict__ slot) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total || slot[i] >= 0) return;   // placed earlier
+    const int c = idx[i], r = rank[i];
+    const int have = filled[(i / n) * k + c];
+    if (r < bf - have) slot[i] = c * bf + have + r;
 }
-__global__ void accept_counts_kernel(const int32_t* __restrict__ start, int bf, long long n_seg,
+__global__ void accept_counts_kernel(const int32_t* __restrict__ count, int bf, long long n_seg,
                                      int32_t* __restrict__ filled) {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n_seg) return;
-    const int cnt = start[c + 1] - start[c], room = bf - filled[c];
+    const int cnt = count[c], room = bf - filled[c];
     filled[c] += cnt < room ? cnt : room;
 }
 
 // per head: exclusive scans of free slots and overflow counts over the centres; `filled` = slots
 // taken in earlier balanced rounds (all zero without them)
 __global__ void __launch_bounds__(1024)
-capacity_scan_kernel(const int32_t* __restrict__ start, const int32_t* __restrict__ filled, int k, int bf,
+capacity_scan_kernel(const int32_t* __restrict__ count, const int32_t* __restrict__ filled, int k, int bf,
                      int32_t* __restrict__ free_base, int32_t* __restrict__ left_base, int32_t* __restrict__ fill_cnt) {
     typedef cub::BlockScan<int, 1024> Scan;
     __shared__ typename Scan::TempStorage tmp;
     __shared__ int s_total_left;
     const int h = blockIdx.x;
-    const int32_t* st = start + (size_t)h * k;
+    const int32_t* ct = count + (size_t)h * k;
     const int32_t* fl = filled + (size_t)h * k;
     int32_t* fb = free_base + (size_t)h * (k + 1);
     int32_t* lb = left_base + (size_t)h * (k + 1);
@@ -432,7 +549,7 @@ capacity_scan_kernel(const int32_t* __restrict__ start, const int32_t* __restric
     for (int c0 = 0; c0 < k; c0 += 1024) {
         const int c = c0 + threadIdx.x;
         int cnt = 0, room = 0;
-        if (c < k) { cnt = st[c + 1] - st[c]; room = bf - fl[c]; }
+        if (c < k) { cnt = ct[c]; room = bf - fl[c]; }
         const int fr = (c < k) ? max(room - cnt, 0) : 0;
         const int lf = (c < k) ? max(cnt - room, 0) : 0;
         int ef, el, tf, tl;
@@ -447,7 +564,7 @@ capacity_scan_kernel(const int32_t* __restrict__ start, const int32_t* __restric
     __syncthreads();
     const int total_left = s_total_left;
     for (int c = threadIdx.x; c < k; c += 1024) {
-        const int cnt = st[c + 1] - st[c], room = bf - fl[c];
+        const int cnt = ct[c], room = bf - fl[c];
         const int fr = max(room - cnt, 0);
         int recv = total_left - fb[c];
         recv = recv < 0 ? 0 : (recv > fr ? fr : recv);
@@ -456,26 +573,22 @@ capacity_scan_kernel(const int32_t* __restrict__ start, const int32_t* __restric
 }
 
 // slot (centre*bf + rank) of every point inside its level (the last round: everything is placed)
-__global__ void placement_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ sorted_ids,
-                                 const int32_t* __restrict__ start, const int32_t* __restrict__ filled,
+__global__ void placement_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ rank,
+                                 const int32_t* __restrict__ count, const int32_t* __restrict__ filled,
                                  const int32_t* __restrict__ free_base, const int32_t* __restrict__ left_base, int n,
-                                 int k, int bf, long long total, long long n_seg, int32_t* __restrict__ slot) {
-    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= total) return;
-    const long long seg = (long long)(keys[j] >> 32);
-    if (seg >= n_seg) return;   // placed in an earlier balanced round
-    const int h = (int)(seg / k);
-    const int c = (int)(seg - (long long)h * k);
-    const int rank = (int)(j - start[seg]);
+                                 int k, int bf, long long total, bool some_placed, int32_t* __restrict__ slot) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total || (some_placed && slot[i] >= 0)) return;   // placed in an earlier balanced round
+    const int h = (int)(i / n);
+    const int c = idx[i], r = rank[i];
     const int32_t* fl = filled + (size_t)h * k;
     const int room = bf - fl[c];
     int s;
-    if (rank < room) {
-        s = c * bf + fl[c] + rank;
+    if (r < room) {
+        s = c * bf + fl[c] + r;
     } else {
         const int32_t* fb = free_base + (size_t)h * (k + 1);
-        const int32_t* st = start + (size_t)h * k;
-        const int L = left_base[(size_t)h * (k + 1) + c] + (rank - room);
+        const int L = left_base[(size_t)h * (k + 1) + c] + (r - room);
         // largest c2 with fb[c2] <= L and a free slot there: upper_bound(fb, L) - 1
         int lo = 0, hi = k;  // search in fb[0..k]
         while (lo < hi) {
@@ -484,10 +597,10 @@ __global__ void placement_kernel(const uint64_t* __restrict__ keys, const uint32
         }
         // skip centres without free slots (fb equal runs): lo is the last index with fb[lo] <= L,
         // which has fb[lo+1] > L, hence at least one free slot
-        const int cnt2 = st[lo + 1] - st[lo];
+        const int cnt2 = count[(size_t)h * k + lo];
         s = lo * bf + fl[lo] + min(cnt2, bf - fl[lo]) + (L - fb[lo]);
     }
-    slot[(size_t)h * n + sorted_ids[j]] = s;
+    slot[i] = s;
 }
 
 // Keys and values of every point to their slot, whole 16-byte pieces.  16 lanes share SCATTER_POINTS points:
@@ -740,9 +853,8 @@ export_kv_kernel(const V* __restrict__ children, int k_pieces, const V* __restri
 // ---------------------------------------------------------------------------
 struct BuildWs {
     size_t total = 0;
-    size_t cents1, cents2, csq, csq_masked, filled, a_idx, a_d2, keys_in, keys_out, vals_in, vals_out, start, fill1,
-        fill2, fbase, lbase, slot1, slot2, cub;
-    size_t cub_bytes = 0;
+    size_t cents1, cents2, csq, csq_masked, filled, a_idx, a_d2, keys, keys2, rank, sorted, start, count, fill1,
+        fill2, fbase, lbase, slot1, slot2;
 };
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -760,22 +872,18 @@ static BuildWs carve(const hira_index_t* ix, int n_keys) {
     w.filled = take(H * k1 * 4);
     w.a_idx = take(H * n * 4);
     w.a_d2 = take(H * n * 4);
-    w.keys_in = take(H * n * 8);
-    w.keys_out = take(H * n * 8);
-    w.vals_in = take(H * n * 4);
-    w.vals_out = take(H * n * 4);
-    w.start = take((H * k1 + 2) * 4);
+    w.keys = take(H * n * 8);
+    w.keys2 = take(H * n * 8);
+    w.rank = take(H * n * 4);
+    w.sorted = take(H * n * 4);
+    w.start = take(H * k1 * 4);
+    w.count = take(H * k1 * 4);
     w.fill1 = take(H * k1 * 4);
     w.fill2 = take(H * k2 * 4);
     w.fbase = take(H * (k1 + 1) * 4);
     w.lbase = take(H * (k1 + 1) * 4);
     w.slot1 = take(H * n * 4);
     w.slot2 = take(H * k1 * 4);
-    size_t cub_bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr,
-                                    (const uint32_t*)nullptr, (uint32_t*)nullptr, (long long)(H * n));
-    w.cub_bytes = cub_bytes;
-    w.cub = take(cub_bytes);
     w.total = off;
     return w;
 }
@@ -791,11 +899,12 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
     float* csq = reinterpret_cast<float*>(base + w.csq);
     int32_t* a_idx = reinterpret_cast<int32_t*>(base + w.a_idx);
     float* a_d2 = reinterpret_cast<float*>(base + w.a_d2);
-    uint64_t* keys_in = reinterpret_cast<uint64_t*>(base + w.keys_in);
-    uint64_t* keys_out = reinterpret_cast<uint64_t*>(base + w.keys_out);
-    uint32_t* vals_in = reinterpret_cast<uint32_t*>(base + w.vals_in);
-    uint32_t* vals_out = reinterpret_cast<uint32_t*>(base + w.vals_out);
+    uint64_t* keys = reinterpret_cast<uint64_t*>(base + w.keys);
+    uint64_t* keys2 = reinterpret_cast<uint64_t*>(base + w.keys2);
+    int32_t* rank = reinterpret_cast<int32_t*>(base + w.rank);
+    uint32_t* sorted = reinterpret_cast<uint32_t*>(base + w.sorted);
     int32_t* start = reinterpret_cast<int32_t*>(base + w.start);
+    int32_t* count = reinterpret_cast<int32_t*>(base + w.count);
     int32_t* fbase = reinterpret_cast<int32_t*>(base + w.fbase);
     int32_t* lbase = reinterpret_cast<int32_t*>(base + w.lbase);
     const int chunks = dim / 8;
@@ -804,28 +913,30 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
         gather_centres_kernel<T><<<grid, 256, 0, s>>>(points, p_head_stride, n, cent_idx, k, dim, cents);
         HIRA_CHECK_LAUNCH("gather centres launch");
     }
-    int seg_bits = 1;
-    while ((1ll << seg_bits) < n_seg) ++seg_bits;
+    const int blocks = (int)((total + 255) / 256);
+    // counts, ranges and ranks of the points' latest assignment; `placed`: the slots of the points to leave out
+    auto sort_members = [&](const int32_t* placed) -> int {
+        cudaMemsetAsync(count, 0, (size_t)n_seg * 4, s);
+        count_members_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, placed, count, rank, status);
+        member_starts_kernel<<<n_heads, 1024, 0, s>>>(count, n, k, start);
+        drop_members_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, start, rank, keys);
+        const long long sblocks = (n_seg + SORT_RANGES - 1) / SORT_RANGES;
+        sort_members_kernel<<<(unsigned)sblocks, SORT_THREADS, 0, s>>>(count, start, n, k, n_seg, keys, keys2, sorted, rank);
+        HIRA_CHECK_LAUNCH("member sort launch");
+        return HIRA_OK;
+    };
     const int iters = n_iters < 1 ? 1 : n_iters;
     for (int it = 0; it < iters; ++it) {
         int rc = run_assign(dtype, points, p_head_stride, cents, csq, n_heads, n, k, dim, use_tc, a_idx, a_d2, s);
         if (rc != HIRA_OK) return rc;
-        const int blocks = (int)((total + 255) / 256);
-        make_sort_keys_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, n_seg, nullptr, keys_in, vals_in, status);
-        HIRA_CHECK_LAUNCH("sort keys launch");
-        size_t cub_bytes = w.cub_bytes;
-        cudaError_t e = cub::DeviceRadixSort::SortPairs(base + w.cub, cub_bytes, keys_in, keys_out, vals_in, vals_out,
-                                                        total, 0, 32 + seg_bits, s);
-        if (e != cudaSuccess) { set_error("radix sort: %s", cudaGetErrorString(e)); return HIRA_ERR_CUDA; }
-        const int blocks1 = (int)((total + 1 + 255) / 256);
-        segment_starts_kernel<<<blocks1, 256, 0, s>>>(keys_out, total, n_seg, start);
-        HIRA_CHECK_LAUNCH("segment starts launch");
+        rc = sort_members(nullptr);
+        if (rc != HIRA_OK) return rc;
         if (it + 1 < iters) {
             const int per_warp = 32 * MeansElem<T>::N;
             const int slabs = (dim + per_warp - 1) / per_warp;
             const long long mblocks = (n_seg * slabs * 32 + 255) / 256;
-            means_kernel<T><<<(unsigned)mblocks, 256, 0, s>>>(points, p_head_stride, n, vals_out, start, k, dim, slabs,
-                                                              n_seg, cents);
+            means_kernel<T><<<(unsigned)mblocks, 256, 0, s>>>(points, p_head_stride, n, sorted, start, count, k, dim,
+                                                              slabs, n_seg, cents);
             HIRA_CHECK_LAUNCH("means launch");
         }
     }
@@ -836,30 +947,21 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
     int32_t* filled = reinterpret_cast<int32_t*>(base + w.filled);
     float* csq_masked = reinterpret_cast<float*>(base + w.csq_masked);
     cudaMemsetAsync(filled, 0, (size_t)n_seg * 4, s);
-    const int blocks = (int)((total + 255) / 256);
     const int seg_blocks = (int)((n_seg + 255) / 256);
     if (balance_rounds > 0) cudaMemsetAsync(slot, 0xff, (size_t)total * 4, s);
     for (int r = 0; r < balance_rounds; ++r) {
-        accept_kernel<<<blocks, 256, 0, s>>>(keys_out, vals_out, start, filled, n, k, bf, total, n_seg, slot);
-        accept_counts_kernel<<<seg_blocks, 256, 0, s>>>(start, bf, n_seg, filled);
+        accept_kernel<<<blocks, 256, 0, s>>>(a_idx, rank, filled, n, k, bf, total, slot);
+        accept_counts_kernel<<<seg_blocks, 256, 0, s>>>(count, bf, n_seg, filled);
         mask_full_centres_kernel<<<seg_blocks, 256, 0, s>>>(csq, filled, bf, n_seg, csq_masked);
         HIRA_CHECK_LAUNCH("balanced round launch");
         int rc = run_assign(dtype, points, p_head_stride, cents, csq_masked, n_heads, n, k, dim, use_tc, a_idx, a_d2, s, true);
         if (rc != HIRA_OK) return rc;
-        make_sort_keys_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, n_seg, slot, keys_in, vals_in, status);
-        HIRA_CHECK_LAUNCH("sort keys launch");
-        size_t cub_bytes = w.cub_bytes;
-        int bits = 1;
-        while ((1ll << bits) <= n_seg) ++bits;   // the sentinel segment n_seg needs one more value
-        cudaError_t e = cub::DeviceRadixSort::SortPairs(base + w.cub, cub_bytes, keys_in, keys_out, vals_in, vals_out,
-                                                        total, 0, 32 + bits, s);
-        if (e != cudaSuccess) { set_error("radix sort: %s", cudaGetErrorString(e)); return HIRA_ERR_CUDA; }
-        segment_starts_kernel<<<(int)((total + 1 + 255) / 256), 256, 0, s>>>(keys_out, total, n_seg, start);
-        HIRA_CHECK_LAUNCH("segment starts launch");
+        rc = sort_members(slot);
+        if (rc != HIRA_OK) return rc;
     }
-    capacity_scan_kernel<<<n_heads, 1024, 0, s>>>(start, filled, k, bf, fbase, lbase, fill);
+    capacity_scan_kernel<<<n_heads, 1024, 0, s>>>(count, filled, k, bf, fbase, lbase, fill);
     HIRA_CHECK_LAUNCH("capacity scan launch");
-    placement_kernel<<<blocks, 256, 0, s>>>(keys_out, vals_out, start, filled, fbase, lbase, n, k, bf, total, n_seg, slot);
+    placement_kernel<<<blocks, 256, 0, s>>>(a_idx, rank, count, filled, fbase, lbase, n, k, bf, total, balance_rounds > 0, slot);
     HIRA_CHECK_LAUNCH("placement launch");
     return HIRA_OK;
 }

@@ -128,6 +128,22 @@ def test_assign_tile_edges(dtype, d, n, k):
     assert np.array_equal(idx.cpu().numpy(), want_i) and np.array_equal(d2.cpu().numpy().view(np.uint32), want_d.view(np.uint32))
 
 
+@pytest.mark.parametrize("n,bf,rounds", [(129, 129, 0), (1000, 1000, 0), (5000, 40, 0), (5000, 40, 2), (13000, 100, 1)])
+def test_build_of_crowded_centres_matches_oracle(n, bf, rounds):
+    """Most points equal, so that one centre has more members than a warp, a block or shared memory sorts."""
+    from util import new_state, random_centres
+    h, d = 2, 16
+    keys = make_keys(h, n, d, 3)
+    keys[:, n // 20:] = keys[:, :1]
+    k1 = -(-n // bf)
+    st = new_state(h, d, bf, 2, k1, torch.float32)
+    c1 = random_centres(h, n, k1, 5)
+    S.build(st, keys, keys.clone(), cent_idx1=c1, n_iters=2, balance_rounds=rounds, use_tensor_cores=False)
+    ox = O.OracleIndex(n_heads=h, dim=d, vdim=d, bf=bf, depth=2, cap_parents=k1, dtype=O.HIRA_F32, vdtype=O.HIRA_F32)
+    O.build(ox, keys, keys.clone(), cent_idx1=c1, n_iters=2, balance_rounds=rounds)
+    assert_index_equal(st, ox, "crowded")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_export_to_unaligned_outputs(dtype):
     st, _, keys, vals = build_both(2, 300, 40, 8, 3, dtype, seed=9)
