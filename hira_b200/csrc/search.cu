@@ -651,7 +651,7 @@ static int launch_search_sc(SearchParams P, int chunks, cudaStream_t stream) {
     P.ring_offset = (uint32_t)off;
     const size_t pieces = (size_t)NCH * (sizeof(T) / 2);
     const size_t smem = off + (size_t)STAGES * RPI * pieces * SEARCH_THREADS * 16;
-    if (smem > 48 * 1024) {
+    if (smem > 44 * 1024) {   // the static arrays come on top
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) {
             set_error("hira_search: cudaFuncSetAttribute(%zu B smem): %s", smem, cudaGetErrorString(e));
@@ -729,6 +729,25 @@ extern "C" int hira_search_tile_parents(const hira_index_t* ix) {
         // small index: one tile, still aligned to grandparent blocks
         tp = ix->depth == 3 ? ((ix->cap_parents + bf - 1) / bf) * bf : ix->cap_parents;
         if (tp * bf > MAX_TILE_ROWS) tp = bf * (MAX_TILE_ROWS / (bf * bf) > 0 ? MAX_TILE_ROWS / (bf * bf) : 1);
+    }
+    // Where the streaming kernel does the search and the tiles leave SMs idle, smaller ones: a tile is walked by
+    // one CTA from its gates to its last row, so with few of them the length of that walk is the time of the
+    // search.  Two CTAs per SM are aimed for, 256 rows are where the fixed part of a CTA takes over.
+    // Measured, whole decode step: 12 heads of 9,001 keys (D = 64, bf = 16) 41.4 us with 1024 rows (108 CTAs),
+    // 39.6 with 512, 35.4 with 256 (432 CTAs), 38.0 with 128.  The int8 pre-filter gains nothing from it
+    // (8 heads of 2,048 keys 27.5, 26.3, 27.4, 30.2 us; 32,768 keys 40.3, 42.3, 46.7, 57.0 us) and keeps its tiles.
+    const bool q8 = ix->children_q8 && ix->dim == 128 && bf >= 8 && (tp * bf) % 128 == 0 && ix->cap_parents % tp == 0;
+    if (!q8 && ix->n_heads >= 1) {
+        auto ctas = [&](int t) { return (long long)ix->n_heads * ((ix->cap_parents + t - 1) / t); };
+        while (ctas(tp) < 2 * 148 && tp * bf > 256) {
+            int next;
+            if (ix->depth == 2) next = (tp + 1) / 2;
+            else if (tp > bf) next = (tp / bf + 1) / 2 * bf;   // whole grandparents
+            else if (tp % 2 == 0) next = tp / 2;               // a divisor of bf
+            else break;
+            if (next == tp) break;
+            tp = next;
+        }
     }
     return tp;
 }

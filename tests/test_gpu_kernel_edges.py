@@ -152,3 +152,19 @@ def test_export_to_unaligned_outputs(dtype):
     L.check(L.load().hira_export(st.struct, 0, 300, out_k.data_ptr(), out_v.data_ptr(), L.current_stream()))
     for out, want in ((out_k, keys), (out_v, vals)):
         assert torch.equal(out[: want.numel() * e].clone(), want.contiguous().view(torch.uint8).flatten())
+
+
+@pytest.mark.parametrize("bf,depth,n,d,heads", [(10, 3, 3000, 128, 2), (16, 2, 9001, 64, 3), (3, 3, 700, 64, 1), (300, 2, 2000, 40, 1),
+                                                (300, 3, 900, 40, 2), (1, 3, 50, 64, 1), (12, 3, 5000, 64, 100)])
+def test_small_tiles_select_what_large_ones_do(bf, depth, n, d, heads):
+    st, _, _, _ = build_both(heads, n, d, bf, depth, torch.bfloat16, seed=61, spare=bf)
+    tp = S.tile_parents(st)
+    assert tp * bf <= 1024 and (depth == 2 or tp % bf == 0 or bf % tp == 0)
+    q = make_queries(heads * 2, d, seed=62)
+    tau = torch.full((heads * 2,), 0.05, device="cuda")
+    large = bf * max(1, 1024 // (bf * bf)) if bf * bf <= 1024 else (1 if depth == 3 else max(1, 1024 // bf))
+    flags = L.HIRA_GATE_GE | L.HIRA_LEAF_GE
+    a = S.search(st, q, tau, flags=flags, want_compact=True)[1].to_lists()
+    b = S.search(st, q, tau, flags=flags, want_compact=True, tp=large)[1].to_lists()
+    for (i, s), (j, t) in zip(a, b):
+        assert torch.equal(i, j) and torch.equal(s, t)
