@@ -20,7 +20,6 @@
 namespace hira {
 
 constexpr int APPEND_THREADS = 512;
-constexpr int APPEND_HW = APPEND_THREADS / GROUP;  // 8-lane groups: one centre row per group per step
 constexpr int APPEND_UNROLL = 4;
 
 struct BestRec;
@@ -32,7 +31,8 @@ struct AppendParams {
     long long k_head_stride, v_head_stride;
     int token_base;
     int32_t* status;
-    // two-kernel path: partial arg-mins of the scan kernel, [head][key][part], or NULL
+    // staged path: partial arg-mins of the scanning CTAs, [head][key][part + 1], or NULL; the last entry of
+    // a key is its nearest grandparent (three levels)
     struct BestRec* partial;
     int n_parts;
     unsigned long long* scan;  // [n_heads] nearest valid parent found by hira_search_scan (n_new == 1), or NULL
@@ -40,12 +40,23 @@ struct AppendParams {
 };
 
 struct BestRec { float s; int i; };
-constexpr int APPEND_MAX_STAGED = 32;  // keys per call the two-kernel path handles
+constexpr int APPEND_MAX_STAGED = 32;  // keys per call the staged path handles
 
 struct Best { float s; int i; };
 
 __device__ __forceinline__ bool better(float s, int i, const Best& b) {
     return s < b.s || (s == b.s && i < b.i);
+}
+
+// the best of a warp's 32 candidates, in every lane (ties: the lower index, so the order does not matter)
+__device__ __forceinline__ Best warp_best(Best b) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        const float s = __shfl_xor_sync(0xffffffffu, b.s, o);
+        const int i = __shfl_xor_sync(0xffffffffu, b.i, o);
+        if (better(s, i, b)) b = Best{s, i};
+    }
+    return b;
 }
 
 // arg-min of sq[p] - 2 x.c_p over p in [0, n) with valid(p); all threads get it.
@@ -89,69 +100,33 @@ __device__ Best nearest_row(const T* rows, const float* sq, int n, const float (
             if (ok[u] && better(s, p, best)) best = Best{s, p};
         }
     }
+    // the 4 groups of a warp (a group agrees), then the warps
+    best = warp_best(best);
     __syncthreads();
-    if (lane == 0) s_best[hw] = best;
+    if ((tid & 31) == 0) s_best[tid >> 5] = best;
     __syncthreads();
-    Best b = s_best[0];
-    for (int w = 1; w < NG; ++w)
-        if (better(s_best[w].s, s_best[w].i, b)) b = s_best[w];
+    Best b = warp_best((tid & 31) < TH / 32 ? s_best[tid & 31] : Best{CUDART_INF_F, 0x7fffffff});
     __syncthreads();
     return b;
 }
 
-// Stage 1 of the two-kernel path: CTA (part, head) scans its slice of the parents that are
-// valid when the call starts, for every new key, and writes one partial arg-min each.  The
-// parents a call creates itself are not in this scan; stage 2 adds them from its own list.
-constexpr int SCAN_THREADS = 256;
-
-template <typename T, int NCH>
-__global__ void __launch_bounds__(SCAN_THREADS, NCH == 2 ? 3 : 1)
-append_scan_kernel(const AppendParams P) {
-    __shared__ Best s_best[SCAN_THREADS / GROUP];
-    const hira_index_t& ix = P.ix;
-    const int h = blockIdx.y, part = blockIdx.x;
-    const int lane = threadIdx.x & (GROUP - 1);
-    const int bf = ix.bf, dim = ix.dim;
-    const size_t capP = ix.cap_parents, capG = ix.cap_gp;
-    const T* parents = reinterpret_cast<const T*>(ix.parents) + (size_t)h * capP * dim;
-    const float* psq = ix.parent_sqnorm + (size_t)h * capP;
-    const int32_t* gc = ix.depth == 3 ? ix.gp_counts + (size_t)h * capG : nullptr;
-    const int32_t* used = ix.used + (size_t)h * 4;
-    const int n_scan = ix.depth == 3 ? used[1] * bf : used[0];
-    const int per = (n_scan + P.n_parts - 1) / P.n_parts;
-    const int lo = min(n_scan, part * per), hi = min(n_scan, lo + per);
-    const T* new_k = reinterpret_cast<const T*>(P.new_k) + (size_t)h * P.k_head_stride;
-    for (int key = 0; key < P.n_new; ++key) {
-        float x[NCH][8];
-        load_vec<T, NCH>(new_k + (size_t)key * dim, x, lane, dim);
-        Best b;
-        if (ix.depth == 3)
-            b = nearest_row<T, NCH, SCAN_THREADS>(parents + (size_t)lo * dim, psq + lo, hi - lo, x, dim,
-                                                  [&](int p) {
-                                                      const int pp = p + lo;
-                                                      const int g = P.bf_magic ? (int)__umulhi((uint32_t)pp, P.bf_magic) : pp / bf;
-                                                      return (pp - g * bf) < gc[g];
-                                                  }, s_best);
-        else
-            b = nearest_row<T, NCH, SCAN_THREADS>(parents + (size_t)lo * dim, psq + lo, hi - lo, x, dim,
-                                                  [&](int) { return true; }, s_best);
-        if (threadIdx.x == 0) {
-            BestRec r;
-            r.s = b.s;
-            r.i = b.i == 0x7fffffff ? b.i : b.i + lo;
-            P.partial[((size_t)h * P.n_new + key) * P.n_parts + part] = r;
-        }
-    }
+__device__ __forceinline__ BestRec load_rec(const BestRec* p) {   // written by other CTAs of the running grid
+    const int2 v = __ldcg(reinterpret_cast<const int2*>(p));
+    BestRec r;
+    r.s = __int_as_float(v.x);
+    r.i = v.y;
+    return r;
 }
 
-template <typename T, typename TV, int NCH, int NVCH>
-__global__ void __launch_bounds__(APPEND_THREADS)
-append_kernel(const AppendParams P) {
-    __shared__ Best s_best[APPEND_HW];
-    __shared__ int s_newp[APPEND_MAX_STAGED];  // parents created earlier in this call (two-kernel path)
-    int n_newp = 0;
+
+// Inserts the keys of head h, one after another; called by a whole CTA.  STAGED: the scans are done and their
+// partial results lie in P.partial; what is left per key is a chain of a few dependent reads.
+template <typename T, typename TV, int NCH, int NVCH, bool STAGED>
+__device__ __forceinline__ void insert_keys(const AppendParams& P, const int h) {
+    __shared__ Best s_best[APPEND_THREADS / 32];
+    __shared__ int s_newp[APPEND_MAX_STAGED], s_newg[APPEND_MAX_STAGED];  // centres created earlier in this call (staged path)
+    int n_newp = 0, n_newg = 0;
     const hira_index_t& ix = P.ix;
-    const int h = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & (GROUP - 1), hw = tid / GROUP;
     const int bf = ix.bf, dim = ix.dim, vdim = ix.vdim;
     const size_t capP = ix.cap_parents, capC = capP * bf, capG = ix.cap_gp;
@@ -178,8 +153,28 @@ append_kernel(const AppendParams P) {
         float x[NCH][8];
         load_vec<T, NCH>(new_k + (size_t)key * dim, x, lane, dim);
 
+        // the better of `b` and the rows listed in s_new (uniform trip count; every group computes the same row)
+        auto nearest_new = [&](const T* rows, const float* sq, const int* s_new, int n_rows, Best b) {
+            for (int e = 0; e < n_rows; ++e) {
+                const int p = s_new[e];
+                Acc2 acc{0.f, 0.f};
+#pragma unroll
+                for (int i = 0; i < NCH; ++i) {
+                    const int c = lane + GROUP * i;
+                    if (c * 8 < dim) {
+                        float a[8];
+                        to_float(load_chunk_coherent<T>(rows + (size_t)p * dim, c), a);
+                        chunk_fma(acc, a, x[i]);
+                    }
+                }
+                const float d = group_sum(__fadd_rn(acc.e, acc.o));
+                const float sc = __fsub_rn(sq[p], __fmul_rn(2.0f, d));
+                if (better(sc, p, b)) b = Best{sc, p};
+            }
+            return b;
+        };
         // ---- nearest valid parent ---------------------------------------------
-        Best bp;
+        Best bp, bg{CUDART_INF_F, 0x7fffffff};
         if (P.scan != nullptr) {
             // found by the search that ran just before on the same index state
             const unsigned long long k = P.scan[h];
@@ -187,29 +182,19 @@ append_kernel(const AppendParams P) {
                               : Best{key_to_float((uint32_t)(k >> 32)), (int)(uint32_t)(k & 0xffffffffu)};
             __syncthreads();                      // every thread has read the slot
             if (tid == 0) P.scan[h] = ~0ull;      // ready for the next search
-        } else if (P.partial != nullptr) {
+        } else if (STAGED) {
             // arg-min over the scanned slices, then over the parents this call created itself
+            const BestRec* pr_ = P.partial + ((size_t)h * P.n_new + key) * (P.n_parts + 1);
             bp = Best{CUDART_INF_F, 0x7fffffff};
-            const BestRec* pr_ = P.partial + ((size_t)h * P.n_new + key) * P.n_parts;
-            for (int s2 = 0; s2 < P.n_parts; ++s2) {
-                const BestRec r = pr_[s2];
+            for (int s2 = tid & 31; s2 < P.n_parts; s2 += 32) {
+                const BestRec r = load_rec(pr_ + s2);
                 if (better(r.s, r.i, bp)) bp = Best{r.s, r.i};
             }
-            for (int e = 0; e < n_newp; ++e) {  // uniform trip count; every group computes the same row
-                const int p = s_newp[e];
-                Acc2 acc{0.f, 0.f};
-#pragma unroll
-                for (int i = 0; i < NCH; ++i) {
-                    const int c = lane + GROUP * i;
-                    if (c * 8 < dim) {
-                        float a[8];
-                        to_float(load_chunk_coherent<T>(parents + (size_t)p * dim, c), a);
-                        chunk_fma(acc, a, x[i]);
-                    }
-                }
-                const float d = group_sum(__fadd_rn(acc.e, acc.o));
-                const float sc = __fsub_rn(psq[p], __fmul_rn(2.0f, d));
-                if (better(sc, p, bp)) bp = Best{sc, p};
+            bp = warp_best(bp);
+            bp = nearest_new(parents, psq, s_newp, n_newp, bp);
+            if (ix.depth == 3) {
+                const BestRec r = load_rec(pr_ + P.n_parts);
+                bg = nearest_new(gps, gsq, s_newg, n_newg, Best{r.s, r.i});
             }
         } else if (ix.depth == 3) {
             const int n_scan = used_g * bf;
@@ -229,7 +214,7 @@ append_kernel(const AppendParams P) {
         if (!placed) {
             if (ix.depth == 3) {
                 // nearest grandparent among those in use (no validity mask: indexer/cuda.py:918-920)
-                const Best bg = nearest_row<T, NCH, APPEND_THREADS>(gps, gsq, used_g, x, dim, [&](int) { return true; }, s_best);
+                if (!STAGED) bg = nearest_row<T, NCH, APPEND_THREADS>(gps, gsq, used_g, x, dim, [&](int) { return true; }, s_best);
                 if (bg.i != 0x7fffffff && gc[bg.i] < bf) {
                     g_dst = bg.i;
                     p_dst = g_dst * bf + gc[g_dst];
@@ -351,29 +336,111 @@ append_kernel(const AppendParams P) {
                 }
             }
         }
-        if (!placed && p_dst >= 0 && P.partial != nullptr && n_newp < APPEND_MAX_STAGED) {
+        if (STAGED && !placed && p_dst >= 0) {   // at most n_new <= APPEND_MAX_STAGED of each
             if (tid == 0) s_newp[n_newp] = p_dst;
             ++n_newp;
+            if (new_gp) {
+                if (tid == 0) s_newg[n_newg] = g_dst;
+                ++n_newg;
+            }
         }
         __syncthreads();  // make the insertion visible to the next key's scan
     }
+}
+
+// The staged path, one launch.  CTA (part, head) scans its slice of the parents that are valid when the call
+// starts, for every new key, and writes one partial arg-min each; the CTA behind the last part does the same
+// over the grandparents.  The CTA of a head that finishes last inserts that head's keys (insert_keys), adding
+// the centres this call creates from its own lists; it is found by a counter in the free fourth word of
+// `used`, which it sets back to zero.  8 heads with 2,048 full parents and 64 grandparents each, the usual
+// state right after a build: 4.9 us scan + 12.5 us insertion a key before, when the insertion was a kernel of
+// 512 threads that each walked the partial list and scanned the grandparents together.
+constexpr int SCAN_THREADS = 256;
+template <typename T, typename TV, int NCH, int NVCH>
+__global__ void __launch_bounds__(SCAN_THREADS, NCH == 2 ? 2 : 1)
+append_staged_kernel(const AppendParams P) {
+    __shared__ int s_last;
+    __shared__ Best s_best[SCAN_THREADS / 32];
+    grid_wait();      // the insertions of the call before
+    grid_trigger();
+    const hira_index_t& ix = P.ix;
+    const int h = blockIdx.y, part = blockIdx.x;
+    const int lane = threadIdx.x & (GROUP - 1);
+    const int bf = ix.bf, dim = ix.dim;
+    const size_t capP = ix.cap_parents, capG = ix.cap_gp;
+    const T* parents = reinterpret_cast<const T*>(ix.parents) + (size_t)h * capP * dim;
+    const float* psq = ix.parent_sqnorm + (size_t)h * capP;
+    const int32_t* gc = ix.depth == 3 ? ix.gp_counts + (size_t)h * capG : nullptr;
+    const int32_t* used = ix.used + (size_t)h * 4;
+    const int n_scan = ix.depth == 3 ? used[1] * bf : used[0];
+    const int per = (n_scan + P.n_parts - 1) / P.n_parts;
+    const int lo = min(n_scan, part * per), hi = min(n_scan, lo + per);
+    const T* new_k = reinterpret_cast<const T*>(P.new_k) + (size_t)h * P.k_head_stride;
+    for (int key = 0; key < P.n_new; ++key) {
+        float x[NCH][8];
+        load_vec<T, NCH>(new_k + (size_t)key * dim, x, lane, dim);
+        Best b;
+        if (part == P.n_parts)   // no validity mask: indexer/cuda.py:918-920
+            b = nearest_row<T, NCH, SCAN_THREADS>(reinterpret_cast<const T*>(ix.grand_parents) + (size_t)h * capG * dim,
+                                                  ix.gp_sqnorm + (size_t)h * capG, used[1], x, dim, [&](int) { return true; }, s_best);
+        else if (ix.depth == 3)
+            b = nearest_row<T, NCH, SCAN_THREADS>(parents + (size_t)lo * dim, psq + lo, hi - lo, x, dim,
+                                                  [&](int p) {
+                                                      const int pp = p + lo;
+                                                      const int g = P.bf_magic ? (int)__umulhi((uint32_t)pp, P.bf_magic) : pp / bf;
+                                                      return (pp - g * bf) < gc[g];
+                                                  }, s_best);
+        else
+            b = nearest_row<T, NCH, SCAN_THREADS>(parents + (size_t)lo * dim, psq + lo, hi - lo, x, dim,
+                                                  [&](int) { return true; }, s_best);
+        if (threadIdx.x == 0) {
+            BestRec r;
+            r.s = b.s;
+            r.i = b.i == 0x7fffffff || part == P.n_parts ? b.i : b.i + lo;
+            P.partial[((size_t)h * P.n_new + key) * (P.n_parts + 1) + part] = r;
+        }
+    }
+    __threadfence();      // the partial results, before the count
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(ix.used + (size_t)h * 4 + 3, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x == 0) ix.used[(size_t)h * 4 + 3] = 0;
+    insert_keys<T, TV, NCH, NVCH, true>(P, h);
+}
+
+template <typename T, typename TV, int NCH, int NVCH>
+__global__ void __launch_bounds__(APPEND_THREADS, 1)
+append_kernel(const AppendParams P) {
+    grid_wait();
+    grid_trigger();
+    insert_keys<T, TV, NCH, NVCH, false>(P, blockIdx.x);
 }
 
 template <typename T, typename TV>
 static int launch_append(const AppendParams& P, cudaStream_t s) {
     const bool k2 = P.ix.dim > 128, v2 = P.ix.vdim > 128;   // chunks per lane: 2 up to 128 elements, else 4
     const int grid = P.ix.n_heads;
+    cudaError_t e = cudaSuccess;
     if (P.partial != nullptr) {
-        dim3 g1((unsigned)P.n_parts, (unsigned)P.ix.n_heads);
-        if (k2) append_scan_kernel<T, 4><<<g1, SCAN_THREADS, 0, s>>>(P);
-        else append_scan_kernel<T, 2><<<g1, SCAN_THREADS, 0, s>>>(P);
-        HIRA_CHECK_LAUNCH("hira_append scan launch");
+        const dim3 g1((unsigned)(P.n_parts + (P.ix.depth == 3 ? 1 : 0)), (unsigned)P.ix.n_heads);
+        auto staged = [&](auto kern) { e = launch_chained(kern, g1, dim3(SCAN_THREADS), 0, s, P); };
+        if (!k2 && !v2) staged(append_staged_kernel<T, TV, 2, 2>);
+        else if (k2 && !v2) staged(append_staged_kernel<T, TV, 4, 2>);
+        else if (!k2 && v2) staged(append_staged_kernel<T, TV, 2, 4>);
+        else staged(append_staged_kernel<T, TV, 4, 4>);
+    } else {
+        auto whole = [&](auto kern) { kern<<<grid, APPEND_THREADS, 0, s>>>(P); e = cudaGetLastError(); };
+        if (!k2 && !v2) whole(append_kernel<T, TV, 2, 2>);
+        else if (k2 && !v2) whole(append_kernel<T, TV, 4, 2>);
+        else if (!k2 && v2) whole(append_kernel<T, TV, 2, 4>);
+        else whole(append_kernel<T, TV, 4, 4>);
     }
-    if (!k2 && !v2) append_kernel<T, TV, 2, 2><<<grid, APPEND_THREADS, 0, s>>>(P);
-    else if (k2 && !v2) append_kernel<T, TV, 4, 2><<<grid, APPEND_THREADS, 0, s>>>(P);
-    else if (!k2 && v2) append_kernel<T, TV, 2, 4><<<grid, APPEND_THREADS, 0, s>>>(P);
-    else append_kernel<T, TV, 4, 4><<<grid, APPEND_THREADS, 0, s>>>(P);
-    HIRA_CHECK_LAUNCH("hira_append launch");
+    if (e != cudaSuccess) {
+        set_error("hira_append launch: %s", cudaGetErrorString(e));
+        return HIRA_ERR_CUDA;
+    }
     return HIRA_OK;
 }
 
@@ -382,8 +449,10 @@ static int launch_append(const AppendParams& P, cudaStream_t s) {
 using namespace hira;
 
 static int append_parts(const hira_index_t* ix) {
-    // enough CTAs to fill the GPU, slices of at least 128 parents
-    int parts = (8 * 148 + ix->n_heads - 1) / ix->n_heads;
+    // two CTAs per SM, all resident at once, where that leaves enough slices; with many heads several waves of
+    // shorter ones; slices of at least 128 parents
+    int parts = 2 * 148 / ix->n_heads - 1;
+    if (parts < 9) parts = (8 * 148 + ix->n_heads - 1) / ix->n_heads < 9 ? (8 * 148 + ix->n_heads - 1) / ix->n_heads : 9;
     const int max_parts = ix->cap_parents / 128;
     if (parts > max_parts) parts = max_parts;
     if (parts > 64) parts = 64;
@@ -392,7 +461,7 @@ static int append_parts(const hira_index_t* ix) {
 
 extern "C" size_t hira_append_workspace_bytes(const hira_index_t* ix, int32_t n_new) {
     if (!ix || n_new < 1 || n_new > APPEND_MAX_STAGED || ix->n_heads < 1 || ix->cap_parents < 1) return 0;
-    return (size_t)ix->n_heads * n_new * append_parts(ix) * sizeof(BestRec);
+    return (size_t)ix->n_heads * n_new * (append_parts(ix) + 1) * sizeof(BestRec);
 }
 
 extern "C" int hira_append(const hira_index_t* ix, const void* new_k, const void* new_v, int32_t n_new,

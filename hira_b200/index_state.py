@@ -131,6 +131,7 @@ class IndexState:
             if src.dtype == torch.uint16 or (dst.dtype == torch.bfloat16 and src.dtype == torch.int16):
                 src = src.view(torch.bfloat16)
             dst.copy_(src.reshape(dst.shape).to(dst.dtype))
+        self.used[:, 3] = 0      # the appends count in it: zero between calls
         self.refresh_int8_copy()
 
     def enable_int8_copy(self, on: bool = True):

@@ -92,7 +92,8 @@ typedef struct hira_index {
     float* gp_sqnorm;      /* [n_heads][cap_gp]                                        */
     int32_t* gp_counts;    /* [n_heads][cap_gp] filled parent slots per grandparent    */
     int32_t* used;         /* [n_heads][4]: {parent slots in use (high-water mark),
-                              grandparents in use, keys stored, reserved}             */
+                              grandparents in use, keys stored, 0: the appends count
+                              their blocks there and leave 0 again}                    */
     /* Optional int8 side copy of the children (dim == 128 only; all three NULL = none).  With it
        hira_search reads 128-byte int8 rows, scores them on the tensor cores and re-reads only the
        rows that can reach the threshold in the index dtype; results are bit-identical.  Written by

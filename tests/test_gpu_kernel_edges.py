@@ -154,6 +154,22 @@ def test_export_to_unaligned_outputs(dtype):
         assert torch.equal(out[: want.numel() * e].clone(), want.contiguous().view(torch.uint8).flatten())
 
 
+@pytest.mark.parametrize("depth,bf,n,d,dtype,m", [(3, 8, 4096, 128, torch.bfloat16, 32), (3, 8, 4096, 64, torch.float32, 9), (3, 8, 2100, 136, torch.bfloat16, 5),
+                                                  (2, 8, 4096, 128, torch.float32, 32), (3, 4, 2048, 16, torch.bfloat16, 33)])
+def test_staged_append_of_several_keys_into_full_parents(depth, bf, n, d, dtype, m):
+    """Every parent is full after the build, so the appended keys open parents and grandparents that the keys
+    behind them in the same call must find; 33 keys take the one-kernel path."""
+    h = 2
+    st, ox, _, _ = build_both(h, n, d, bf, depth, dtype, seed=31, spare=bf * 40)
+    assert (L.load().hira_append_workspace_bytes(st.struct, m) > 0) == (m <= 32)
+    for r in range(2):
+        nk, nv = make_keys(h, m, d, 40 + r, dtype), make_keys(h, m, d, 50 + r, dtype, normalize=False)
+        nk[:, m // 2:] = nk[:, : m - m // 2]       # twins: the second goes under the parent the first opened
+        S.append(st, nk, nv)
+        O.append(ox, nk, nv)
+    assert_index_equal(st, ox, "staged append")
+
+
 @pytest.mark.parametrize("bf,depth,n,d,heads", [(10, 3, 3000, 128, 2), (16, 2, 9001, 64, 3), (3, 3, 700, 64, 1), (300, 2, 2000, 40, 1),
                                                 (300, 3, 900, 40, 2), (1, 3, 50, 64, 1), (12, 3, 5000, 64, 100)])
 def test_small_tiles_select_what_large_ones_do(bf, depth, n, d, heads):
