@@ -76,9 +76,10 @@ def hira_decode_attention(query: torch.Tensor, cache_output, *, scaling: Optiona
     b, hq, lq, d = query.shape
     if lq != 1:
         raise NotImplementedError("hira_decode_attention handles one query token per step")
-    q = query.reshape(b * hq, d)
+    q = query
     if q.device != st.device or q.dtype not in (torch.float32, torch.bfloat16):
         q = q.to(device=st.device, dtype=torch.float32)
+    q = q.view(b * hq, d) if q.is_contiguous() else q.reshape(b * hq, d).contiguous()
     sm_scale = float(scaling) if scaling is not None else d ** -0.5
     bufs = getattr(searcher, "_decode_bufs", None)
     if bufs is None or bufs[0].shape != (b * hq, d) or bufs[0].device != st.device:
@@ -100,16 +101,19 @@ def hira_decode_attention(query: torch.Tensor, cache_output, *, scaling: Optiona
     qk = cache_output.queued_keys
     queued_k = queued_v = None
     if qk is not None and qk.shape[-2] > 0:
-        queued_k = qk.reshape(-1, qk.shape[-2], qk.shape[-1]).to(st.dtype).contiguous()
         qv = cache_output.queued_values
-        queued_v = qv.reshape(-1, qv.shape[-2], qv.shape[-1]).to(st.vdtype).contiguous()
+        queued_k, queued_v = qk, qv
+        stride = S.queue_stride(qk) if qk.dtype == st.dtype and qk.device == st.device else None
+        if stride is None or qv.dtype != st.vdtype or qv.device != st.device or S.queue_stride(qv) != stride:
+            # not the filled part of two like queue buffers: a dense copy
+            queued_k = qk.reshape(-1, qk.shape[-2], qk.shape[-1]).to(st.dtype).contiguous()
+            queued_v = qv.reshape(-1, qv.shape[-2], qv.shape[-1]).to(st.vdtype).contiguous()
     n_splits = S.attn_splits(st, n_q, compact.tile_parents)
     ws = getattr(srch, "_attn_ws", None)
     need = n_q * n_splits * (st.vdim + 2)
     if ws is None or ws.numel() < need or ws.device != st.device:
         ws = srch._attn_ws = torch.empty((need,), dtype=torch.float32, device=st.device)
     out = torch.empty((n_q, st.vdim), dtype=torch.float32, device=st.device)
-    q = q.contiguous()
     scan_key = scan_out = None
     if append_key is not None:
         if q2kv is not None:

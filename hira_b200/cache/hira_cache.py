@@ -105,9 +105,17 @@ class HiraCacheLayer(CacheLayerMixin):
                             indexer=self.indexer, searcher=self.searcher),
                 None,
             )
-        self._enqueue(key_states, value_states)
-        if self.queued_len >= self.update_every:
-            self.update_index()
+        n = key_states.shape[-2]
+        if (self.queued_len == 0 and n >= self.update_every and key_states.dtype == self.dtype
+                and value_states.dtype == self.vdtype and key_states.device == self.device == value_states.device
+                and key_states.shape[:2] == value_states.shape[:2] == self._queue_k.shape[:2]):
+            # nothing waits and a flush is due: straight into the index, without a copy through the queue
+            self.indexer.update(key_states, value_states)
+            self.indexed_len += n
+        else:
+            self._enqueue(key_states, value_states)
+            if self.queued_len >= self.update_every:
+                self.update_index()
         return (
             CacheOutput(queued_keys=self.queued_keys, queued_values=self.queued_values,
                         prefill_keys=None, prefill_values=None,

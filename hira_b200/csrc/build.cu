@@ -1075,9 +1075,28 @@ static int build_impl(const hira_index_t* ix, const void* keys_v, const void* va
     return q8_refresh(ix, s, ix->depth == 3 ? (long long)k2 * bf : (long long)k1);
 }
 
+// point drawn by u in [0, 1) out of stride c of k equal strides of n points
+__global__ void stratified_kernel(const float* __restrict__ u, int n, int k, long long total, int32_t* __restrict__ out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const long long c = i % k, lo = c * n / k, width = (c + 1) * n / k - lo;
+    long long j = (long long)__fmul_rn(u[i], (float)width);
+    const long long last = width > 1 ? width - 1 : 0;
+    out[i] = (int32_t)(lo + (j < last ? j : last));
+}
+
 }  // namespace hira
 
 using namespace hira;
+
+extern "C" int hira_stratified(const float* u, int32_t n_heads, int32_t n, int32_t k, int32_t* out, void* stream) {
+    HIRA_CHECK_ARG(u && out, HIRA_ERR_ARG, "hira_stratified: NULL argument");
+    HIRA_CHECK_ARG(n_heads >= 1 && n >= 1 && k >= 1, HIRA_ERR_SHAPE, "hira_stratified: n_heads=%d n=%d k=%d", n_heads, n, k);
+    const long long total = (long long)n_heads * k;
+    stratified_kernel<<<(unsigned)((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(u, n, k, total, out);
+    HIRA_CHECK_LAUNCH("hira_stratified launch");
+    return HIRA_OK;
+}
 
 extern "C" size_t hira_build_workspace_bytes(const hira_index_t* ix, int32_t n_keys) {
     if (validate_index(ix, false) != HIRA_OK || n_keys < 0) return 0;

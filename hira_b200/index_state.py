@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -70,6 +71,7 @@ class IndexState:
             self.children_q8 = self.children_q8_meta = self.q8_chan_scale = self.q8_query_scratch = None
         self.status = z((1,), dtype=torch.int32, device=dev)
         self._struct = None
+        self._append_bytes = {}
         self._active_parents = 0
         self.refresh_struct()
 
@@ -92,6 +94,7 @@ class IndexState:
         for name in self.ARRAYS + self.Q8_ARRAYS:
             setattr(s, name, L.ptr(getattr(self, name)))
         self._struct = s
+        self._byref = C.byref(s)
         return s
 
     @property
@@ -105,12 +108,14 @@ class IndexState:
         n = int(n)
         if n < 0 or n >= self.cap_parents:
             n = 0
+        if n == self._active_parents:
+            return
         self._active_parents = n
         self._struct.active_parents = n
 
     @property
     def struct(self):
-        return C.byref(self._struct)
+        return self._byref
 
     def state_dict(self) -> dict:
         d = {name: getattr(self, name) for name in self.ARRAYS if getattr(self, name) is not None}
@@ -269,10 +274,37 @@ def alloc_compact(st: IndexState, hq: int, tp: Optional[int] = None) -> CompactR
         tile_parents=tp, tile_rows=tp * st.bf)
 
 
+@lru_cache(maxsize=256)
+def _default_splits(hq: int, tiles: int) -> int:   # a pure function of the two numbers
+    return int(L.load().hira_attn_default_splits(hq, tiles))
+
+
 def attn_splits(st: IndexState, hq: int, tp: Optional[int] = None) -> int:
     tp = tp or tile_parents(st)
     tiles = n_tiles(st, tp) if st.active_parents == 0 else -(-st.active_parents // tp)
-    return int(L.load().hira_attn_default_splits(hq, tiles))
+    return _default_splits(hq, tiles)
+
+
+def queue_stride(t: torch.Tensor) -> Optional[int]:
+    """Elements between the heads of a (B, H, n, D) or (H, n, D) queue whose rows lie one behind another from
+    a 16-byte boundary -- a whole tensor or the filled part of a queue buffer --, None for any other layout."""
+    d, strides = t.shape[-1], t.stride()
+    hs = strides[-3]
+    if strides[-1] != 1 or strides[-2] != d or hs < t.shape[-2] * d or t.data_ptr() % 16 or hs * t.element_size() % 16:
+        return None
+    if t.ndim == 4 and t.shape[0] > 1 and strides[0] != t.shape[1] * hs:
+        return None
+    return hs
+
+
+def _queue_layout(st: IndexState, queued_k: torch.Tensor, queued_v: torch.Tensor):
+    """(queued keys per head, elements between the heads): one stride serves both arrays."""
+    assert queued_k.dtype == st.dtype and queued_v.dtype == st.vdtype
+    if st.vdim != st.dim:
+        raise ValueError("queued keys/values with vdim != dim are not supported")
+    stride = queue_stride(queued_k)
+    assert stride is not None and stride == queue_stride(queued_v)
+    return queued_k.shape[-2], stride
 
 
 def sparse_attn(st: IndexState, q, scaling, compact: CompactResult, *, q2kv=None, queued_k=None, queued_v=None,
@@ -289,12 +321,7 @@ def sparse_attn(st: IndexState, q, scaling, compact: CompactResult, *, q2kv=None
         out = torch.empty((hq, st.vdim), dtype=torch.float32, device=dev)
     n_queued, qstride = 0, 0
     if queued_k is not None and queued_k.shape[-2] > 0:
-        assert queued_k.is_contiguous() and queued_v.is_contiguous()
-        assert queued_k.dtype == st.dtype and queued_v.dtype == st.vdtype
-        n_queued = queued_k.shape[-2]
-        qstride = n_queued * st.dim
-        if st.vdim != st.dim:
-            raise ValueError("queued keys/values with vdim != dim are not supported")
+        n_queued, qstride = _queue_layout(st, queued_k, queued_v)
     rc = lib.hira_sparse_attn(st.struct, L.ptr(q), L.ptr(scaling), L.ptr(q2kv), hq, compact.tile_parents,
                               L.ptr(compact.idx), L.ptr(compact.score), L.ptr(compact.count),
                               L.ptr(queued_k) if n_queued else None, L.ptr(queued_v) if n_queued else None,
@@ -329,7 +356,10 @@ def append(st: IndexState, new_k: torch.Tensor, new_v: Optional[torch.Tensor], t
         assert new_v.is_contiguous() and new_v.dtype == st.vdtype
     ws, nbytes = None, 0
     if use_workspace:
-        nbytes = int(lib.hira_append_workspace_bytes(st.struct, m))
+        sizes = st._append_bytes     # depends on the heads, the capacity and m only
+        nbytes = sizes.get(m)
+        if nbytes is None:
+            nbytes = sizes[m] = int(lib.hira_append_workspace_bytes(st.struct, m))
         if nbytes:
             ws = getattr(st, "_append_ws", None)
             if ws is None or ws.numel() < nbytes:
@@ -398,12 +428,7 @@ def decode_attention(st: IndexState, q: torch.Tensor, sm_scale: float, tau: torc
     hq = q.shape[0]
     n_queued, qstride = 0, 0
     if queued_k is not None and queued_k.shape[-2] > 0:
-        assert queued_k.is_contiguous() and queued_v.is_contiguous()
-        assert queued_k.dtype == st.dtype and queued_v.dtype == st.vdtype
-        n_queued = queued_k.shape[-2]
-        qstride = n_queued * st.dim
-        if st.vdim != st.dim:
-            raise ValueError("queued keys/values with vdim != dim are not supported")
+        n_queued, qstride = _queue_layout(st, queued_k, queued_v)
     rest = (L.ptr(q2kv), hq, max_group, flags, compact.tile_parents, L.ptr(q_hat), L.ptr(logit_scale),
             L.ptr(compact.idx), L.ptr(compact.score), L.ptr(compact.count),
             L.ptr(queued_k) if n_queued else None, L.ptr(queued_v) if n_queued else None,
@@ -451,6 +476,14 @@ def build(st: IndexState, keys: torch.Tensor, values: Optional[torch.Tensor], *,
                         n_iters, int(balance_rounds), 1 if use_tensor_cores else 0, L.ptr(st.status), L.ptr(ws), nbytes,
                         L.current_stream(st.device))
     L.check(rc, "hira_build")
+
+
+def stratified(u: torch.Tensor, n: int) -> torch.Tensor:
+    """u (H, k) in [0, 1) -> (H, k) int32: the point u draws out of each of k equal strides of n points."""
+    h, k = u.shape
+    out = torch.empty((h, k), dtype=torch.int32, device=u.device)
+    L.check(L.load().hira_stratified(L.ptr(u), h, n, k, L.ptr(out), L.current_stream(u.device)), "hira_stratified")
+    return out
 
 
 def recompute_radii(st: IndexState):

@@ -131,12 +131,18 @@ class CUDAIndexer(BaseIndexer):
         b, h, l, d = t.shape
         return t.reshape(b * h, l, d).contiguous()
 
+    def _rows(self, t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+        """(B, H, M, D) as contiguous (B*H, M, D) rows of the index's device and `dtype`."""
+        if t.dtype != dtype or t.device != self.state.device or not t.is_contiguous():
+            return self._fold(t.to(self.state.device)).to(dtype)
+        if t.ndim != 4:
+            raise ValueError(f"expected a (B, H, L, D) tensor, got {tuple(t.shape)}")
+        return t.view(-1, t.shape[2], t.shape[3]) if t.shape[0] != 1 else t[0]
+
     @staticmethod
     def _stratified(h: int, n: int, k: int, g: torch.Generator, device) -> torch.Tensor:
-        lo = (torch.arange(k + 1, device=device, dtype=torch.int64) * n) // k        # stride boundaries
-        width = (lo[1:] - lo[:-1]).to(torch.float32)
-        jitter = (torch.rand((h, k), generator=g, device=device) * width).to(torch.int64)
-        return (lo[:-1] + torch.minimum(jitter, (lo[1:] - lo[:-1] - 1).clamp_min(0))).to(torch.int32).contiguous()
+        u = torch.rand((h, k), generator=g, device=device)     # one point out of each of k equal strides
+        return S.stratified(u, n)
 
     def _capacity_parents(self, n_keys: int) -> int:
         bf = self.branching_factor
@@ -308,27 +314,27 @@ class CUDAIndexer(BaseIndexer):
         assert new_values is None or new_keys.shape[:3] == new_values.shape[:3]
         if new_keys.ndim != 4:
             raise ValueError(f"new_keys must be (B, H, M, D), got {tuple(new_keys.shape)}")
-        k = self._fold(new_keys.to(self.state.device))
-        h, m, d = k.shape
-        if h != self.num_heads or d != self.dim:
-            raise ValueError(f"new_keys has (heads, dim)=({h}, {d}), index has ({self.num_heads}, {self.dim})")
-        has_values = self.state.values is not None
+        st = self.state
+        b, hk, m, d = new_keys.shape
+        if b * hk != self.num_heads or d != self.dim:
+            raise ValueError(f"new_keys has (heads, dim)=({b * hk}, {d}), index has ({self.num_heads}, {self.dim})")
+        k = self._rows(new_keys, st.dtype)
         v = None
-        if has_values:
+        if st.values is not None:
             if new_values is None:
                 raise ValueError("the index stores values: new_values is required")
-            v = self._fold(new_values.to(self.state.device)).to(self.state.vdtype)
+            v = self._rows(new_values, st.vdtype)
         if m == 0:
             return self
         self._ensure_capacity(m)
         if scanned:
             if m != 1 or not self._scan_pending:
                 raise ValueError("update(scanned=True) needs one key per head and a search that scanned for it")
-            S.append_scanned(self.state, k.to(self.state.dtype), v, self._scan_slots)
+            S.append_scanned(self.state, k, v, self._scan_slots)
         else:
             if self._scan_pending:
                 self._scan_slots.fill_(-1)    # the index changes: that scan is void
-            S.append(self.state, k.to(self.state.dtype), v)
+            S.append(self.state, k, v)
         self._scan_pending = False
         self._parents_bound += m
         self._gp_bound += m

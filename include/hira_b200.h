@@ -432,6 +432,10 @@ int hira_kth_score(const hira_index_t* index, int32_t n_qheads,
                    void* stream);
 
 /* ------------------------------------------------------------------------- */
+/* Initial centres of a build: out[h][c] = the point that u[h][c] in [0, 1) draws out of stride c of k equal
+ * strides of n points (device pointers). */
+int hira_stratified(const float* u, int32_t n_heads, int32_t n, int32_t k, int32_t* out, void* stream);
+
 /* Build.  Replaces CUDAIndexer.build (indexer/cuda.py:56-108) with its
  * helpers (:114-538): per level, nearest-centroid assignment, capacity-bf
  * grouping closest-first with overflow into free slots, blocked layout,

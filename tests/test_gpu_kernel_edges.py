@@ -184,3 +184,35 @@ def test_small_tiles_select_what_large_ones_do(bf, depth, n, d, heads):
     b = S.search(st, q, tau, flags=flags, want_compact=True, tp=large)[1].to_lists()
     for (i, s), (j, t) in zip(a, b):
         assert torch.equal(i, j) and torch.equal(s, t)
+
+
+@pytest.mark.parametrize("b,cap,n", [(1, 16, 5), (2, 16, 1), (2, 7, 7), (1, 4, 3)])
+@pytest.mark.parametrize("how", ["buffer", "transposed", "other_dtype"])
+def test_queue_views_attend_like_dense_queues(b, cap, n, how):
+    """The filled part of a queue buffer is attended in place, any other layout through a copy."""
+    from hira_b200 import CacheOutput, CUDAIndexer, CUDASearcher, hira_decode_attention
+    h, d = 3, 64
+    g = torch.Generator().manual_seed(cap)
+    mk = lambda *s: torch.randn(s, generator=g).to(torch.bfloat16).cuda()   # noqa: E731
+    ix = CUDAIndexer(3, 1, 16).build(mk(b, h, 600, d), mk(b, h, 600, d))
+    q, tau = mk(b, h * 2, 1, d), torch.full((b * h * 2,), 1.5, device="cuda")
+    qk, qv = mk(b, h, cap, d), mk(b, h, cap, d)
+    if how == "transposed":
+        view = lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)[:, :, :n]   # noqa: E731
+    elif how == "other_dtype":
+        view = lambda t: t.float()[:, :, :n]   # noqa: E731
+    else:
+        view = lambda t: t[:, :, :n]   # noqa: E731
+    outs = [hira_decode_attention(q, CacheOutput(k, v, None, None, ix, CUDASearcher()), threshold=tau)
+            for k, v in ((view(qk), view(qv)), (qk[:, :, :n].contiguous(), qv[:, :, :n].contiguous()))]
+    assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("h,n,k", [(1, 1, 1), (3, 1000, 7), (2, 5, 5), (8, 131072, 4096)])
+def test_stratified_centres(h, n, k):
+    u = torch.rand((h, k), generator=torch.Generator(device="cuda").manual_seed(n), device="cuda")
+    u[0, 0] = 1.0 - 2.0 ** -24
+    lo = (torch.arange(k + 1, device="cuda", dtype=torch.int64) * n) // k
+    width = lo[1:] - lo[:-1]
+    want = lo[:-1] + torch.minimum((u * width.float()).to(torch.int64), (width - 1).clamp_min(0))
+    assert torch.equal(S.stratified(u, n), want.to(torch.int32))
