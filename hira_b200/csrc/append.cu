@@ -238,7 +238,10 @@ __device__ __forceinline__ void insert_keys(const AppendParams& P, const int h) 
             if constexpr (NCH == 2) {
                 if (ix.children_q8 != nullptr) {
                     const size_t at = (size_t)h * capC + slot;
-                    q8_write_row(x, ix.q8_chan_scale + (size_t)h * HIRA_Q8_CHAN,
+                    const float* chan = ix.q8_chan_scale + (size_t)h * HIRA_Q8_CHAN;
+                    float inv[2][8];
+                    q8_load_inv_scales(chan, inv, lane);
+                    q8_write_row(x, inv, chan, q8_slack(chan),
                                  reinterpret_cast<int8_t*>(ix.children_q8) + at * 128,
                                  reinterpret_cast<uint32_t*>(ix.children_q8_meta) + at, slot & 7, lane);
                 }

@@ -407,60 +407,128 @@ __device__ __forceinline__ void load_vec(const T* v, float (&b)[NCH][8], int lan
 // ---------------------------------------------------------------------------
 // int8 side copy of a child row (D = 128), written by the 8 lanes of a group; see search_q8.cu.
 //   x        the lane's two chunks of the row in fp32 (values exactly as stored in the index)
-//   chan     per-channel scales s_i [128] followed by min_i s_i at [128]
+//   chan     per-channel scales s_i [128]; inv: 1 / s_i of the lane's channels; slack: 2^-15 / min_i s_i
 //   dst      the row's 128 bytes;  swz = slot & 7 permutes its 16-byte chunks
 //   meta     (step, err) as two fp16: k'_i = x_i / s_i, step = max |k'_i| / 127 rounded up, k~_i = rint(k'_i / step),
 //            err >= ||k' - step k~||_2 + 2^-15 ||x||_2 / min_i s_i  (the second term covers the
 //            rounding of the canonical fp32 dot product for any query: ||q (.) s|| >= min s ||q||)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void q8_write_row(const float (&x)[2][8], const float* __restrict__ chan, int8_t* dst,
-                                             uint32_t* meta, int swz, int lane) {
-    float kp[2][8];
-    float amax = 0.f;
-    Acc2 nx{0.f, 0.f};
+// Both quotients are defined as correctly rounded divisions, but a division per element and quotient was
+// most of the quantisation's time.  So they are formed with reciprocals (of the scales once for all rows of
+// a group, of the step once a row), which is within 4e-7 of the quotient, and divided out only where that
+// could round differently: a step whose fp16 neighbours are in question, a quotient next to half an integer.
+// The stored step and integers are those of the divisions; err takes the residual of the k' at hand, whose
+// own rounding (2^-22 of ||q|| ||x|| at most) lies far inside its second term.
+// v[0..15] (the lane's two chunks of a row) divided by their scales and then by step; out of line, because 32
+// divisions in the rows' loop would push it out of the instruction cache for the sake of a few rows
+__device__ __noinline__ static void q8_divide(float* v, const float* chan, int lane, float step) {
+#pragma unroll 1
+    for (int t = 0; t < 16; ++t) {
+        const float s = __ldg(chan + 8 * (lane + GROUP * (t >> 3)) + (t & 7));
+        v[t] = __fdiv_rn(__fdiv_rn(v[t], s), step);
+    }
+}
+__device__ __forceinline__ void q8_quotients(const float (&x)[2][8], const float* chan, int lane, float step, float (&out)[2][8]) {
+    float v[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) v[t] = x[t >> 3][t & 7];
+    q8_divide(v, chan, lane, step);
+#pragma unroll
+    for (int t = 0; t < 16; ++t) out[t >> 3][t & 7] = v[t];
+}
+__device__ __forceinline__ void q8_load_inv_scales(const float* __restrict__ chan, float (&inv)[2][8], int lane) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int c = lane + GROUP * i;
         const float4 s0 = __ldg(reinterpret_cast<const float4*>(chan) + 2 * c);
         const float4 s1 = __ldg(reinterpret_cast<const float4*>(chan) + 2 * c + 1);
-        const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        inv[i][0] = s0.x; inv[i][1] = s0.y; inv[i][2] = s0.z; inv[i][3] = s0.w;
+        inv[i][4] = s1.x; inv[i][5] = s1.y; inv[i][6] = s1.z; inv[i][7] = s1.w;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            kp[i][e] = __fdiv_rn(x[i][e], sc[e]);
-            amax = fmaxf(amax, fabsf(kp[i][e]));
-        }
+        for (int e = 0; e < 8; ++e) inv[i][e] = __fdiv_rn(1.0f, inv[i][e]);
+    }
+}
+// the factor of ||x|| in err
+__device__ __forceinline__ float q8_slack(const float* __restrict__ chan) { return __fdiv_ru(3.1e-5f, __ldg(chan + 128)); }
+// rounded to the nearest integer (ties to even) and its low byte, for |t| < 2^22: no conversion unit involved
+constexpr float Q8_ROUND = 12582912.0f;   // 1.5 * 2^23
+__device__ __forceinline__ float q8_row_max(const float (&kp)[2][8]) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(kp[i][e]));
+    const unsigned gm = group_mask();
+    m = fmaxf(m, __shfl_xor_sync(gm, m, 4));
+    m = fmaxf(m, __shfl_xor_sync(gm, m, 2));
+    return fmaxf(m, __shfl_xor_sync(gm, m, 1));
+}
+__device__ __forceinline__ void q8_write_row(const float (&x)[2][8], const float (&inv)[2][8],
+                                             const float* __restrict__ chan, float slack, int8_t* dst, uint32_t* meta,
+                                             int swz, int lane) {
+    float kp[2][8];
+    Acc2 nx{0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) kp[i][e] = __fmul_rn(x[i][e], inv[i][e]);
         chunk_fma(nx, x[i], x[i]);
     }
-    const unsigned gm = group_mask();
-    amax = fmaxf(amax, __shfl_xor_sync(gm, amax, 4));
-    amax = fmaxf(amax, __shfl_xor_sync(gm, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(gm, amax, 1));
+    float amax = q8_row_max(kp);
     // the step is stored as fp16, so it is rounded (up) to one first and the row quantised with that
+    __half h_step = __float2half_ru(amax * ((1.0f / 127.0f) * (1.0f + 6e-7f)));
+    if (__half_as_ushort(h_step) != __half_as_ushort(__float2half_ru(amax * ((1.0f / 127.0f) * (1.0f - 6e-7f))))) {   // the same in the 8 lanes
+        q8_quotients(x, chan, lane, 1.0f, kp);
+        amax = q8_row_max(kp);
+        h_step = __float2half_ru(__fdiv_rn(amax, 127.0f));
+    }
     bool ok = amax > 0.f && amax < 3.0e38f;
-    float step = ok ? __half2float(__float2half_ru(__fdiv_rn(amax, 127.0f))) : 1.0f;
+    float step = ok ? __half2float(h_step) : 1.0f;
     if (!(step > 0.f) || !(step < 6.0e4f)) { ok = false; step = 1.0f; }
+    const float inv_step = ok ? __fdiv_rn(1.0f, step) : 0.f;
+    float kr[2][8];    // the quotients rounded, plus Q8_ROUND; within +-127 because the step was rounded up
+    float off = 0.f;   // how far from an integer the farthest quotient lies
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float t = __fmul_rn(kp[i][e], inv_step);
+            kr[i][e] = __fadd_rn(t, Q8_ROUND);
+            off = fmaxf(off, fabsf(__fsub_rn(t, __fsub_rn(kr[i][e], Q8_ROUND))));
+        }
+    }
+    if (off > 0.49995f && ok) {   // the quotients are off by 127 x 4e-7 at most: divide what lies that close to a tie
+        q8_quotients(x, chan, lane, step, kr);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) kr[i][e] = __fadd_rn(kr[i][e], Q8_ROUND);
+    }
     Acc2 ne{0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         float dlt[8];
-        uint32_t w[2] = {0u, 0u};
+        uint32_t w[2];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            float kq = ok ? rintf(__fdiv_rn(kp[i][e], step)) : 0.f;
-            kq = fminf(fmaxf(kq, -127.f), 127.f);
-            dlt[e] = __fmaf_rn(-kq, step, kp[i][e]);
-            w[e >> 2] |= ((uint32_t)(int)kq & 0xffu) << (8 * (e & 3));
+        for (int e = 0; e < 8; ++e) dlt[e] = __fmaf_rn(-__fsub_rn(kr[i][e], Q8_ROUND), step, kp[i][e]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t lo = __byte_perm(__float_as_uint(kr[i][4 * j]), __float_as_uint(kr[i][4 * j + 1]), 0x0040);
+            const uint32_t hi = __byte_perm(__float_as_uint(kr[i][4 * j + 2]), __float_as_uint(kr[i][4 * j + 3]), 0x0040);
+            w[j] = ok ? __byte_perm(lo, hi, 0x5410) : 0u;
         }
         chunk_fma(ne, dlt, dlt);
         const int c = lane + GROUP * i;        // 8-element chunk of the row: half (c & 1) of 16-byte chunk c >> 1
-        const int off = (((c >> 1) ^ swz) << 4) + ((c & 1) << 3);
-        *reinterpret_cast<uint2*>(dst + off) = make_uint2(w[0], w[1]);
+        const int off8 = (((c >> 1) ^ swz) << 4) + ((c & 1) << 3);
+        *reinterpret_cast<uint2*>(dst + off8) = make_uint2(w[0], w[1]);
     }
     const float err2 = group_sum(__fadd_rn(ne.e, ne.o));
     const float xsq = group_sum(__fadd_rn(nx.e, nx.o));
     if (lane == 0) {
-        const float min_s = __ldg(chan + 128);
-        const float err = ok ? sqrtf(err2) * 1.001f + 3.1e-5f * sqrtf(xsq) / min_s
+        // square roots by the reciprocal's unit: 2 ulp, inside the 1.001 and the room of the slack
+        const float e1 = err2 > 0.f ? err2 * rsqrtf(err2) : err2;                     // finite where it is used
+        const float x1 = xsq > 0.f && xsq < 3.0e38f ? xsq * rsqrtf(xsq) : xsq;        // an overflow stays infinite
+        const float err = ok ? e1 * 1.001f + slack * x1
                              : (amax > 0.f ? 3.0e38f : 0.f);    // a row that cannot be quantised is always a candidate
         // rounded up; beyond the fp16 range it becomes +inf, which keeps the row a candidate
         *meta = (uint32_t)__half_as_ushort(__float2half_ru(step)) | ((uint32_t)__half_as_ushort(__float2half_ru(err)) << 16);
