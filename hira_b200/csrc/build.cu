@@ -436,11 +436,13 @@ sort_members_kernel(const int32_t* __restrict__ cnt, const int32_t* __restrict__
 
 // Lloyd mean update.  The members of a centre are added one after another in sorted order, so a centre is
 // a serial chain; what it must not be is a chain of memory latencies.  One warp owns a slab of the
-// channels of one centre (32 of fp32, 64 of bf16: one 128-byte piece of every member row) and keeps
-// MEANS_FLIGHT member rows in flight ahead of the additions; the ids of the next batch are fetched beside
-// them.  Measured, 8 x 4,096 fp32 keys of 128 channels, 64 centres: 42.1 -> 17.2 us (one 8-lane group per
-// centre with one row in flight before).
-constexpr int MEANS_FLIGHT = 32;
+// channels of one centre (32 of fp32, 64 of bf16: one 128-byte piece of every member row) and keeps a ring of
+// STAGES batches of 32 member rows in flight in shared memory ahead of the additions (each lane reads
+// only what it copied itself).  Random centres have hubs -- thousands of members after the first assignment --
+// and the longest chain is the time of the kernel.  8 x 4,096 fp32 keys of 128 channels, 64 centres: 42.1 us
+// a call on average with one row of an 8-lane group in flight, 17.6 us with 32 rows in registers; with the ring
+// a build of ten such iterations went from 950 to 850 us.
+constexpr int MEANS_BATCH = 32, MEANS_WARPS = 4;
 template <typename T> struct MeansElem;
 template <> struct MeansElem<float> {
     typedef float raw; static constexpr int N = 1;
@@ -458,15 +460,16 @@ template <> struct MeansElem<__nv_bfloat16> {
         return *reinterpret_cast<const uint32_t*>(&p);
     }
 };
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int STAGES>
+__global__ void __launch_bounds__(MEANS_WARPS * 32)
 means_kernel(const T* __restrict__ points, long long p_head_stride, int n, const uint32_t* __restrict__ sorted_ids,
              const int32_t* __restrict__ start, const int32_t* __restrict__ count, int k, int dim, int slabs,
              long long n_seg, T* __restrict__ cents) {
     typedef MeansElem<T> E;
     typedef typename E::raw raw_t;
-    const int wl = threadIdx.x & 31;
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    extern __shared__ __align__(16) uint32_t ring_all[];
+    const int wl = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long w = (long long)blockIdx.x * MEANS_WARPS + warp;
     const long long seg = w / slabs;
     if (seg >= n_seg) return;   // the whole warp
     const int d = ((int)(w - seg * slabs) * 32 + wl) * E::N;
@@ -475,28 +478,56 @@ means_kernel(const T* __restrict__ points, long long p_head_stride, int n, const
     if (e <= b) return;  // empty cluster keeps its centre
     const bool on = d < dim;
     const T* P = points + (size_t)h * p_head_stride + (on ? d : 0);
+    uint32_t* ring = ring_all + warp * (STAGES * MEANS_BATCH * 32) + wl;   // [stage][row][lane]
+    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
     float sum[E::N];
 #pragma unroll
     for (int j = 0; j < E::N; ++j) sum[j] = 0.f;
-    uint32_t ids = b + wl < e ? sorted_ids[b + wl] : 0u;
-    for (int m = b; m < e; m += MEANS_FLIGHT) {   // uniform over the warp
-        const uint32_t next = m + MEANS_FLIGHT + wl < e ? sorted_ids[m + MEANS_FLIGHT + wl] : 0u;
-        raw_t r[MEANS_FLIGHT];
+    const int batches = (e - b + MEANS_BATCH - 1) / MEANS_BATCH;   // uniform over the warp, as every test below
+    auto load_ids = [&](int t) { const int m = b + t * MEANS_BATCH + wl; return m < e ? sorted_ids[m] : 0u; };
+    auto issue = [&](int t, uint32_t ids) {
+        if (t < batches) {
+            const int np = min(MEANS_BATCH, e - b - t * MEANS_BATCH);
+            const uint32_t dst = ring_s + (uint32_t)(t % STAGES) * (MEANS_BATCH * 128);
 #pragma unroll
-        for (int u = 0; u < MEANS_FLIGHT; ++u) {
-            const uint32_t id = __shfl_sync(0xffffffffu, ids, u);
-            if (m + u < e) r[u] = __ldg(reinterpret_cast<const raw_t*>(P + (size_t)id * dim));
+            for (int u = 0; u < MEANS_BATCH; ++u) {
+                const uint32_t id = __shfl_sync(0xffffffffu, ids, u);
+                if (u < np)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + u * 128), "l"(P + (size_t)id * dim) : "memory");
+            }
         }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    uint32_t ids = load_ids(0);
 #pragma unroll
-        for (int u = 0; u < MEANS_FLIGHT; ++u) {
-            if (m + u < e) {
+    for (int t = 0; t < STAGES - 1; ++t) {
+        const uint32_t next = load_ids(t + 1);
+        issue(t, ids);
+        ids = next;
+    }
+    for (int t = 0; t < batches; ++t) {
+        const uint32_t next = load_ids(t + STAGES);
+        issue(t + STAGES - 1, ids);
+        ids = next;
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 1) : "memory");
+        const int np = min(MEANS_BATCH, e - b - t * MEANS_BATCH);
+        const uint32_t* src = ring + (t % STAGES) * (MEANS_BATCH * 32);
+        if (np == MEANS_BATCH) {
+#pragma unroll
+            for (int u = 0; u < MEANS_BATCH; ++u) {
                 float a[E::N];
-                E::get(r[u], a);
+                E::get(reinterpret_cast<const raw_t*>(src)[u * 32], a);
+#pragma unroll
+                for (int j = 0; j < E::N; ++j) sum[j] = __fadd_rn(sum[j], a[j]);
+            }
+        } else {
+            for (int u = 0; u < np; ++u) {
+                float a[E::N];
+                E::get(reinterpret_cast<const raw_t*>(src)[u * 32], a);
 #pragma unroll
                 for (int j = 0; j < E::N; ++j) sum[j] = __fadd_rn(sum[j], a[j]);
             }
         }
-        ids = next;
     }
     if (!on) return;
     const float cnt = (float)(e - b);
@@ -934,9 +965,18 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
         if (it + 1 < iters) {
             const int per_warp = 32 * MeansElem<T>::N;
             const int slabs = (dim + per_warp - 1) / per_warp;
-            const long long mblocks = (n_seg * slabs * 32 + 255) / 256;
-            means_kernel<T><<<(unsigned)mblocks, 256, 0, s>>>(points, p_head_stride, n, sorted, start, count, k, dim,
-                                                              slabs, n_seg, cents);
+            const long long mblocks = (n_seg * slabs + MEANS_WARPS - 1) / MEANS_WARPS;
+            auto means = [&](auto kern, int stages) -> int {
+                const int smem = MEANS_WARPS * stages * MEANS_BATCH * 128;
+                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                if (e != cudaSuccess) { set_error("means: cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return HIRA_ERR_CUDA; }
+                kern<<<(unsigned)mblocks, MEANS_WARPS * 32, smem, s>>>(points, p_head_stride, n, sorted, start, count, k, dim, slabs,
+                                                                       n_seg, cents);
+                return HIRA_OK;
+            };
+            // crowded centres: a deep ring for their chains; many small ones: twice the warps per SM instead
+            rc = n >= 48ll * k ? means(means_kernel<T, 4>, 4) : means(means_kernel<T, 2>, 2);
+            if (rc != HIRA_OK) return rc;
             HIRA_CHECK_LAUNCH("means launch");
         }
     }
