@@ -53,7 +53,8 @@ __device__ __forceinline__ void memcpy_chunk(RawChunk<T>& raw, const T* src) {
 constexpr int SQ_THREADS = 64;
 template <typename T>
 __global__ void __launch_bounds__(SQ_THREADS)
-sqnorm_seq_kernel(const T* __restrict__ rows, long long n_rows, int dim, float* __restrict__ out) {
+sqnorm_seq_kernel(const T* __restrict__ rows, long long n_rows, int dim, float* __restrict__ out,
+                  int32_t* __restrict__ zero) {
     const long long i = (long long)blockIdx.x * SQ_THREADS + threadIdx.x;
     if (i >= n_rows) return;
     constexpr int FLIGHT = 16 / (int)sizeof(T);   // 8-element chunks: 128 bytes of bf16, 128 of fp32
@@ -80,6 +81,7 @@ sqnorm_seq_kernel(const T* __restrict__ rows, long long n_rows, int dim, float* 
         }
     }
     out[i] = acc;
+    if (zero) zero[i] = 0;   // the centre's member count, for the assignment that follows
 }
 
 // ---------------------------------------------------------------------------
@@ -229,14 +231,14 @@ static int launch_assign_cc(const T* points, long long p_head_stride, const T* c
 
 static int run_assign(int dtype, const void* points, long long p_head_stride, const void* cents, float* csq,
                       int n_heads, int n, int k, int dim, int use_tc, int32_t* out_idx, float* out_d2,
-                      cudaStream_t s, bool csq_ready = false) {
+                      cudaStream_t s, bool csq_ready = false, int32_t* zero = nullptr) {
     const long long rows = (long long)n_heads * k;
     const int blocks = (int)((rows + SQ_THREADS - 1) / SQ_THREADS);
     if (!csq_ready) {
         if (dtype == HIRA_BF16)
-            sqnorm_seq_kernel<<<blocks, SQ_THREADS, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(cents), rows, dim, csq);
+            sqnorm_seq_kernel<<<blocks, SQ_THREADS, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(cents), rows, dim, csq, zero);
         else
-            sqnorm_seq_kernel<<<blocks, SQ_THREADS, 0, s>>>(reinterpret_cast<const float*>(cents), rows, dim, csq);
+            sqnorm_seq_kernel<<<blocks, SQ_THREADS, 0, s>>>(reinterpret_cast<const float*>(cents), rows, dim, csq, zero);
         HIRA_CHECK_LAUNCH("sqnorm launch");
     }
     if (use_tc && assign_tc_supported(dtype, n, k, dim))
@@ -251,6 +253,12 @@ static int run_assign(int dtype, const void* points, long long p_head_stride, co
 // ---------------------------------------------------------------------------
 // Level build pieces.
 // ---------------------------------------------------------------------------
+// chunk c (8 elements) of a row; rows of a build lie on 16-byte boundaries
+template <typename T>
+__device__ __forceinline__ void copy_chunk(T* dst, const T* src, int c) {
+    reinterpret_cast<RawChunk<T>*>(dst)[c] = load_chunk<T>(src, c);
+}
+
 template <typename T>
 __global__ void gather_centres_kernel(const T* __restrict__ points, long long p_head_stride, int n,
                                       const int32_t* __restrict__ cent_idx, int k, int dim, T* __restrict__ cents) {
@@ -267,10 +275,7 @@ __global__ void gather_centres_kernel(const T* __restrict__ points, long long p_
     } else {
         src = (int)(((long long)c * n) / k);  // evenly strided
     }
-    const T* r = points + (size_t)h * p_head_stride + (size_t)src * dim + ch * 8;
-    T* w = cents + ((size_t)h * k + c) * dim + ch * 8;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) w[e] = r[e];
+    copy_chunk(cents + ((size_t)h * k + c) * dim, points + (size_t)h * p_head_stride + (size_t)src * dim, ch);
 }
 
 // ---------------------------------------------------------------------------
@@ -564,7 +569,7 @@ __global__ void accept_counts_kernel(const int32_t* __restrict__ count, int bf, 
 }
 
 // per head: exclusive scans of free slots and overflow counts over the centres; `filled` = slots
-// taken in earlier balanced rounds (all zero without them)
+// taken in earlier balanced rounds (NULL without them)
 __global__ void __launch_bounds__(1024)
 capacity_scan_kernel(const int32_t* __restrict__ count, const int32_t* __restrict__ filled, int k, int bf,
                      int32_t* __restrict__ free_base, int32_t* __restrict__ left_base, int32_t* __restrict__ fill_cnt) {
@@ -573,14 +578,14 @@ capacity_scan_kernel(const int32_t* __restrict__ count, const int32_t* __restric
     __shared__ int s_total_left;
     const int h = blockIdx.x;
     const int32_t* ct = count + (size_t)h * k;
-    const int32_t* fl = filled + (size_t)h * k;
+    auto fl = [&](int c) { return filled ? filled[(size_t)h * k + c] : 0; };
     int32_t* fb = free_base + (size_t)h * (k + 1);
     int32_t* lb = left_base + (size_t)h * (k + 1);
     int carry_f = 0, carry_l = 0;
     for (int c0 = 0; c0 < k; c0 += 1024) {
         const int c = c0 + threadIdx.x;
         int cnt = 0, room = 0;
-        if (c < k) { cnt = ct[c]; room = bf - fl[c]; }
+        if (c < k) { cnt = ct[c]; room = bf - fl(c); }
         const int fr = (c < k) ? max(room - cnt, 0) : 0;
         const int lf = (c < k) ? max(cnt - room, 0) : 0;
         int ef, el, tf, tl;
@@ -595,11 +600,11 @@ capacity_scan_kernel(const int32_t* __restrict__ count, const int32_t* __restric
     __syncthreads();
     const int total_left = s_total_left;
     for (int c = threadIdx.x; c < k; c += 1024) {
-        const int cnt = ct[c], room = bf - fl[c];
+        const int cnt = ct[c], room = bf - fl(c);
         const int fr = max(room - cnt, 0);
         int recv = total_left - fb[c];
         recv = recv < 0 ? 0 : (recv > fr ? fr : recv);
-        fill_cnt[(size_t)h * k + c] = fl[c] + min(cnt, room) + recv;
+        fill_cnt[(size_t)h * k + c] = fl(c) + min(cnt, room) + recv;
     }
 }
 
@@ -612,11 +617,11 @@ __global__ void placement_kernel(const int32_t* __restrict__ idx, const int32_t*
     if (i >= total || (some_placed && slot[i] >= 0)) return;   // placed in an earlier balanced round
     const int h = (int)(i / n);
     const int c = idx[i], r = rank[i];
-    const int32_t* fl = filled + (size_t)h * k;
-    const int room = bf - fl[c];
+    auto fl = [&](int x) { return filled ? filled[(size_t)h * k + x] : 0; };
+    const int room = bf - fl(c);
     int s;
     if (r < room) {
-        s = c * bf + fl[c] + r;
+        s = c * bf + fl(c) + r;
     } else {
         const int32_t* fb = free_base + (size_t)h * (k + 1);
         const int L = left_base[(size_t)h * (k + 1) + c] + (r - room);
@@ -629,7 +634,7 @@ __global__ void placement_kernel(const int32_t* __restrict__ idx, const int32_t*
         // skip centres without free slots (fb equal runs): lo is the last index with fb[lo] <= L,
         // which has fb[lo+1] > L, hence at least one free slot
         const int cnt2 = count[(size_t)h * k + lo];
-        s = lo * bf + fl[lo] + min(cnt2, bf - fl[lo]) + (L - fb[lo]);
+        s = lo * bf + fl(lo) + min(cnt2, bf - fl(lo)) + (L - fb[lo]);
     }
     slot[i] = s;
 }
@@ -687,10 +692,7 @@ __global__ void scatter_parents_kernel(const T* __restrict__ cents1, const int32
     if (t >= (long long)k1 * chunks) return;
     const int c = (int)(t / chunks), ch = (int)(t % chunks);
     const int s = slot2 ? slot2[(size_t)h * k1 + c] : c;
-    const T* r8 = cents1 + ((size_t)h * k1 + c) * dim + ch * 8;
-    T* w8 = parents + ((size_t)h * cap_parents + s) * dim + ch * 8;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) w8[e] = r8[e];
+    copy_chunk(parents + ((size_t)h * cap_parents + s) * dim, cents1 + ((size_t)h * k1 + c) * dim, ch);
     if (ch == 0) child_counts[(size_t)h * cap_parents + s] = fill1[(size_t)h * k1 + c];
 }
 
@@ -702,10 +704,7 @@ __global__ void scatter_gps_kernel(const T* __restrict__ cents2, const int32_t* 
     const int h = blockIdx.y;
     if (t >= (long long)k2 * chunks) return;
     const int g = (int)(t / chunks), ch = (int)(t % chunks);
-    const T* r8 = cents2 + ((size_t)h * k2 + g) * dim + ch * 8;
-    T* w8 = gps + ((size_t)h * cap_gp + g) * dim + ch * 8;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) w8[e] = r8[e];
+    copy_chunk(gps + ((size_t)h * cap_gp + g) * dim, cents2 + ((size_t)h * k2 + g) * dim, ch);
     if (ch == 0) gp_counts[(size_t)h * cap_gp + g] = fill2[(size_t)h * k2 + g];
 }
 
@@ -947,7 +946,7 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
     const int blocks = (int)((total + 255) / 256);
     // counts, ranges and ranks of the points' latest assignment; `placed`: the slots of the points to leave out
     auto sort_members = [&](const int32_t* placed) -> int {
-        cudaMemsetAsync(count, 0, (size_t)n_seg * 4, s);
+        if (placed) cudaMemsetAsync(count, 0, (size_t)n_seg * 4, s);   // else cleared with the norms of the centres
         count_members_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, placed, count, rank, status);
         member_starts_kernel<<<n_heads, 1024, 0, s>>>(count, n, k, start);
         drop_members_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, start, rank, keys);
@@ -958,7 +957,7 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
     };
     const int iters = n_iters < 1 ? 1 : n_iters;
     for (int it = 0; it < iters; ++it) {
-        int rc = run_assign(dtype, points, p_head_stride, cents, csq, n_heads, n, k, dim, use_tc, a_idx, a_d2, s);
+        int rc = run_assign(dtype, points, p_head_stride, cents, csq, n_heads, n, k, dim, use_tc, a_idx, a_d2, s, false, count);
         if (rc != HIRA_OK) return rc;
         rc = sort_members(nullptr);
         if (rc != HIRA_OK) return rc;
@@ -986,9 +985,12 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
     // rule, indexer/cuda.py:252-334) goes to the free slots in (centre, distance) order.
     int32_t* filled = reinterpret_cast<int32_t*>(base + w.filled);
     float* csq_masked = reinterpret_cast<float*>(base + w.csq_masked);
-    cudaMemsetAsync(filled, 0, (size_t)n_seg * 4, s);
     const int seg_blocks = (int)((n_seg + 255) / 256);
-    if (balance_rounds > 0) cudaMemsetAsync(slot, 0xff, (size_t)total * 4, s);
+    if (balance_rounds > 0) {
+        cudaMemsetAsync(filled, 0, (size_t)n_seg * 4, s);
+        cudaMemsetAsync(slot, 0xff, (size_t)total * 4, s);
+    }
+    const int32_t* taken = balance_rounds > 0 ? filled : nullptr;   // NULL: every centre starts empty
     for (int r = 0; r < balance_rounds; ++r) {
         accept_kernel<<<blocks, 256, 0, s>>>(a_idx, rank, filled, n, k, bf, total, slot);
         accept_counts_kernel<<<seg_blocks, 256, 0, s>>>(count, bf, n_seg, filled);
@@ -999,9 +1001,9 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
         rc = sort_members(slot);
         if (rc != HIRA_OK) return rc;
     }
-    capacity_scan_kernel<<<n_heads, 1024, 0, s>>>(count, filled, k, bf, fbase, lbase, fill);
+    capacity_scan_kernel<<<n_heads, 1024, 0, s>>>(count, taken, k, bf, fbase, lbase, fill);
     HIRA_CHECK_LAUNCH("capacity scan launch");
-    placement_kernel<<<blocks, 256, 0, s>>>(a_idx, rank, count, filled, fbase, lbase, n, k, bf, total, balance_rounds > 0, slot);
+    placement_kernel<<<blocks, 256, 0, s>>>(a_idx, rank, count, taken, fbase, lbase, n, k, bf, total, balance_rounds > 0, slot);
     HIRA_CHECK_LAUNCH("placement launch");
     return HIRA_OK;
 }
