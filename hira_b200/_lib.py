@@ -26,7 +26,7 @@ EXPORTED_SYMBOLS = [
     "hira_append_workspace_bytes",
     "hira_threshold", "hira_kth_score", "hira_prepare_query", "hira_build_workspace_bytes", "hira_build",
     "hira_recompute_radii", "hira_export", "hira_assign", "hira_sparse_attn_noalloc", "hira_decode_attention",
-    "hira_decode_attention_sampled", "hira_stratified",
+    "hira_decode_attention_sampled", "hira_stratified", "hira_grow",
     "hira_search_scan", "hira_append_scanned", "hira_step_events_create", "hira_step_events_destroy",
     "hira_decode_step", "hira_q8_refresh", "hira_q8_fallback_count",
     "hira_exchange_bytes", "hira_peer_alloc", "hira_peer_open", "hira_peer_close", "hira_peer_free", "hira_exchange_merge",
@@ -137,6 +137,8 @@ def _declare(lib):
     lib.hira_build.argtypes = [IX, P, P, I32, I64, I64, I32, P, P, I32, I32, I32, P, P, SZ, P]
     lib.hira_stratified.restype = C.c_int
     lib.hira_stratified.argtypes = [P, I32, I32, I32, P, P]
+    lib.hira_grow.restype = C.c_int
+    lib.hira_grow.argtypes = [IX, IX, P]
     lib.hira_q8_refresh.restype = C.c_int
     lib.hira_q8_refresh.argtypes = [IX, P]
     lib.hira_recompute_radii.restype = C.c_int

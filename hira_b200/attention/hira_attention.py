@@ -41,8 +41,8 @@ def _samples_for(indexer, sample_size: int) -> torch.Tensor:
     filled = st.slot2token >= 0                                   # (H, capC)
     # random filled slots per head: top-s of random scores masked to filled slots
     r = torch.rand(filled.shape, generator=g, device=st.device).masked_fill_(~filled, -1.0)
-    n_filled = int(filled.sum(dim=1).min().item())
-    s = max(1, min(s, n_filled))
+    if getattr(indexer, "_built_keys", 0) < s:      # a build stores all its keys and nothing removes one
+        s = max(1, min(s, int(filled.sum(dim=1).min().item())))
     slots = r.topk(s, dim=1).indices                              # (H, s)
     rows = st.children.gather(1, slots.unsqueeze(-1).expand(-1, -1, st.dim)).contiguous()
     indexer._tau_samples = (st, rows)

@@ -445,8 +445,8 @@ sort_members_kernel(const int32_t* __restrict__ cnt, const int32_t* __restrict__
 // STAGES batches of 32 member rows in flight in shared memory ahead of the additions (each lane reads
 // only what it copied itself).  Random centres have hubs -- thousands of members after the first assignment --
 // and the longest chain is the time of the kernel.  8 x 4,096 fp32 keys of 128 channels, 64 centres: 42.1 us
-// a call on average with one row of an 8-lane group in flight, 17.6 us with 32 rows in registers; with the ring
-// a build of ten such iterations went from 950 to 850 us.
+// a call on average with one row of an 8-lane group in flight, 17.6 us with 32 rows in registers, 9.8 us
+// with the ring.
 constexpr int MEANS_BATCH = 32, MEANS_WARPS = 4;
 template <typename T> struct MeansElem;
 template <> struct MeansElem<float> {
@@ -1117,6 +1117,29 @@ static int build_impl(const hira_index_t* ix, const void* keys_v, const void* va
     return q8_refresh(ix, s, ix->depth == 3 ? (long long)k2 * bf : (long long)k1);
 }
 
+// ---------------------------------------------------------------------------
+// A larger copy of an index: every head's part of every array copied and the room behind it filled, all arrays
+// in one launch (a copy and a fill per array before, some forty launches of a few microseconds).
+// ---------------------------------------------------------------------------
+struct GrowItem { const char* src; char* dst; long long src_bytes, dst_bytes; uint32_t fill; };   // bytes per head
+constexpr int GROW_ITEMS = 16;
+struct GrowItems { GrowItem it[GROW_ITEMS]; };
+__global__ void __launch_bounds__(256)
+grow_kernel(const GrowItems items) {
+    const GrowItem g = items.it[blockIdx.z];
+    const char* src = g.src + (size_t)blockIdx.y * g.src_bytes;
+    char* dst = g.dst + (size_t)blockIdx.y * g.dst_bytes;
+    const long long first = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+    if ((((uintptr_t)src | (uintptr_t)dst | (uintptr_t)g.src_bytes | (uintptr_t)g.dst_bytes) & 15) == 0) {
+        const uint4 f = make_uint4(g.fill, g.fill, g.fill, g.fill);
+        for (long long i = first; i < g.dst_bytes / 16; i += step)
+            reinterpret_cast<uint4*>(dst)[i] = i < g.src_bytes / 16 ? reinterpret_cast<const uint4*>(src)[i] : f;
+    } else {   // the arrays of single words, where a head's part may start at any of them
+        for (long long i = first; i < g.dst_bytes / 4; i += step)
+            reinterpret_cast<uint32_t*>(dst)[i] = i < g.src_bytes / 4 ? reinterpret_cast<const uint32_t*>(src)[i] : g.fill;
+    }
+}
+
 // point drawn by u in [0, 1) out of stride c of k equal strides of n points
 __global__ void stratified_kernel(const float* __restrict__ u, int n, int k, long long total, int32_t* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1130,6 +1153,45 @@ __global__ void stratified_kernel(const float* __restrict__ u, int n, int k, lon
 }  // namespace hira
 
 using namespace hira;
+
+extern "C" int hira_grow(const hira_index_t* from, const hira_index_t* to, void* stream) {
+    int rc = validate_index(from, false);
+    if (rc == HIRA_OK) rc = validate_index(to, false);
+    if (rc != HIRA_OK) return rc;
+    HIRA_CHECK_ARG(from->dtype == to->dtype && from->vdtype == to->vdtype && from->depth == to->depth && from->bf == to->bf &&
+                   from->dim == to->dim && from->vdim == to->vdim && from->n_heads == to->n_heads, HIRA_ERR_SHAPE,
+                   "hira_grow: the two indexes differ in more than their capacity");
+    HIRA_CHECK_ARG(from->cap_parents <= to->cap_parents, HIRA_ERR_CAPACITY, "hira_grow: capacity %d does not fit into %d",
+                   from->cap_parents, to->cap_parents);
+    HIRA_CHECK_ARG(to->n_heads <= 65535, HIRA_ERR_SHAPE, "hira_grow: %d heads exceed the grid limit", to->n_heads);
+    GrowItems items;
+    int n = 0;
+    auto add = [&](const void* src, void* dst, long long row, long long rows_from, long long rows_to, uint32_t fill) {
+        if (src && dst) items.it[n++] = GrowItem{(const char*)src, (char*)dst, row * rows_from, row * rows_to, fill};
+    };
+    const long long es = (long long)elem_size(to->dtype), ves = (long long)elem_size(to->vdtype), p0 = from->cap_parents,
+                    p1 = to->cap_parents, c0 = p0 * to->bf, c1 = p1 * to->bf, g0 = from->cap_gp, g1 = to->cap_gp;
+    add(from->children, to->children, to->dim * es, c0, c1, 0);
+    add(from->values, to->values, to->vdim * ves, c0, c1, 0);
+    add(from->slot2token, to->slot2token, 4, c0, c1, 0xffffffffu);
+    add(from->parents, to->parents, to->dim * es, p0, p1, 0);
+    add(from->parent_radii, to->parent_radii, 4, p0, p1, 0);
+    add(from->parent_sqnorm, to->parent_sqnorm, 4, p0, p1, 0);
+    add(from->child_counts, to->child_counts, 4, p0, p1, 0);
+    if (to->depth == 3) {
+        add(from->grand_parents, to->grand_parents, to->dim * es, g0, g1, 0);
+        add(from->gp_radii, to->gp_radii, 4, g0, g1, 0);
+        add(from->gp_sqnorm, to->gp_sqnorm, 4, g0, g1, 0);
+        add(from->gp_counts, to->gp_counts, 4, g0, g1, 0);
+    }
+    add(from->used, to->used, 4, 4, 4, 0);
+    add(from->children_q8, to->children_q8, 128, c0, c1, 0);
+    add(from->children_q8_meta, to->children_q8_meta, 4, c0, c1, 0);
+    add(from->q8_chan_scale, to->q8_chan_scale, 4, HIRA_Q8_CHAN, HIRA_Q8_CHAN, 0);
+    grow_kernel<<<dim3(64, (unsigned)to->n_heads, (unsigned)n), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(items);
+    HIRA_CHECK_LAUNCH("hira_grow launch");
+    return HIRA_OK;
+}
 
 extern "C" int hira_stratified(const float* u, int32_t n_heads, int32_t n, int32_t k, int32_t* out, void* stream) {
     HIRA_CHECK_ARG(u && out, HIRA_ERR_ARG, "hira_stratified: NULL argument");

@@ -154,7 +154,14 @@ class IndexState:
         """A copy with more parent slots (and grandparent slots); existing slots keep their positions."""
         new = IndexState(n_heads=self.n_heads, dim=self.dim, vdim=self.vdim, bf=self.bf, depth=self.depth,
                          cap_parents=new_cap_parents, dtype=self.dtype, vdtype=self.vdtype, device=self.device,
-                         with_values=self.values is not None, int8_copy=self.int8_copy)
+                         with_values=self.values is not None, int8_copy=self.int8_copy, cleared=self.device.type != "cuda")
+        new.status.copy_(self.status)
+        if self.device.type == "cuda":
+            old = L.HiraIndexStruct.from_buffer_copy(self._struct)
+            for name in self.Q8_ARRAYS:     # also when enable_int8_copy has left them out of the view
+                setattr(old, name, L.ptr(getattr(self, name)))
+            L.check(L.load().hira_grow(C.byref(old), new.struct, L.current_stream(self.device)), "hira_grow")
+            return new
         for name in self.ARRAYS + self.Q8_ARRAYS:
             src = getattr(self, name)
             if src is None or name == "used":
@@ -164,7 +171,6 @@ class IndexState:
                 continue
             getattr(new, name)[:, : src.shape[1]].copy_(src)
         new.used.copy_(self.used)
-        new.status.copy_(self.status)
         return new
 
 

@@ -72,6 +72,7 @@ class CUDAIndexer(BaseIndexer):
         self._pinned = None
         self._appended = 0        # keys appended since the build
         self._n_keys = 0
+        self._built_keys = 0      # keys of the latest build: every head holds at least as many
 
     # ---- reference attribute names as views ---------------------------------
     @property
@@ -210,7 +211,7 @@ class CUDAIndexer(BaseIndexer):
         S.build(st, keys, values, cent_idx1=cent1, cent_idx2=cent2, n_iters=max(1, int(self.max_iterations)),
                 balance_rounds=self.balance_rounds, use_tensor_cores=self.use_tensor_cores)
         self.state = st
-        self._n_keys = n
+        self._n_keys = self._built_keys = n
         self._parents_bound = k2 * bf if st.depth == 3 else k1
         self._gp_bound = k2
         self._snapshot = None

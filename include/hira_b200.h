@@ -432,6 +432,10 @@ int hira_kth_score(const hira_index_t* index, int32_t n_qheads,
                    void* stream);
 
 /* ------------------------------------------------------------------------- */
+/* Copies an index into one of the same shape and a larger capacity whose arrays need not be cleared: slots keep
+ * their positions, the room behind them is left free. */
+int hira_grow(const hira_index_t* from, const hira_index_t* to, void* stream);
+
 /* Initial centres of a build: out[h][c] = the point that u[h][c] in [0, 1) draws out of stride c of k equal
  * strides of n points (device pointers). */
 int hira_stratified(const float* u, int32_t n_heads, int32_t n, int32_t k, int32_t* out, void* stream);

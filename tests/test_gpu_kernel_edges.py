@@ -216,3 +216,23 @@ def test_stratified_centres(h, n, k):
     width = lo[1:] - lo[:-1]
     want = lo[:-1] + torch.minimum((u * width.float()).to(torch.int64), (width - 1).clamp_min(0))
     assert torch.equal(S.stratified(u, n), want.to(torch.int32))
+
+
+
+@pytest.mark.parametrize("depth,bf,d,cap_extra,dtype,vals", [(3, 8, 128, 8, torch.bfloat16, True), (2, 7, 64, 3, torch.float32, False),
+                                                             (2, 5, 128, 1, torch.float32, True), (3, 1, 8, 6, torch.bfloat16, True)])
+def test_grown_state_keeps_its_slots_and_leaves_the_rest_free(depth, bf, d, cap_extra, dtype, vals):
+    h, n = 3, 50 * bf + 1
+    st, _, _, _ = build_both(h, n, d, bf, depth, dtype, seed=17, spare=bf, with_values=vals)
+    torch.full((1 << 24,), 0x5A, dtype=torch.uint8, device="cuda")      # what the allocator hands out next is not zero
+    new = st.grown(st.cap_parents + cap_extra)
+    assert new.cap_parents >= st.cap_parents + cap_extra
+    for name in S.IndexState.ARRAYS + ("children_q8", "children_q8_meta", "q8_chan_scale"):
+        a, b = getattr(st, name), getattr(new, name)
+        if a is None:
+            continue
+        m = a.shape[1]
+        assert torch.equal(a.view(torch.uint8), b[:, :m].contiguous().view(torch.uint8)), name
+        if name not in ("used", "q8_chan_scale"):
+            rest = b[:, m:].contiguous()
+            assert torch.equal(rest, torch.full_like(rest, -1 if name == "slot2token" else 0)), name
