@@ -95,9 +95,7 @@ def hira_decode_attention(query: torch.Tensor, cache_output, *, scaling: Optiona
     if hasattr(indexer, "wait_pending_update"):
         indexer.wait_pending_update()                            # an update still running on a side stream
     st.active_parents = getattr(indexer, "active_parents", 0)   # empty capacity is not visited
-    compact = srch._compact
-    if compact is None or compact.idx.device != st.device or tuple(compact.idx.shape) != (n_q, st.cap_children):
-        compact = srch._compact = S.alloc_compact(st, n_q)
+    compact = srch._compact = S.compact_for(st, n_q, srch._compact)
     qk = cache_output.queued_keys
     queued_k = queued_v = None
     if qk is not None and qk.shape[-2] > 0:

@@ -203,7 +203,7 @@ class CompactResult:
 
 def tile_parents(st: IndexState) -> int:
     tp = getattr(st, "_tile_parents", None)
-    if tp is None:   # depends on bf, depth and the capacity only: fixed for the life of the state
+    if tp is None:   # depends on bf, depth, capacity, heads and whether the int8 copy is in use now; kept from then on
         tp = st._tile_parents = int(L.load().hira_search_tile_parents(st.struct))
     return tp
 
@@ -227,8 +227,10 @@ def search(st: IndexState, q: torch.Tensor, tau: torch.Tensor, *, scaling=None, 
     also scored against that key for the `append_scanned` that follows."""
     lib = L.load()
     hq = q.shape[0]
-    tp = tp or tile_parents(st)
-    if want_compact and compact is None:
+    tp = tp or (tile_parents(st) if compact is None else compact.tile_parents)
+    if compact is not None:
+        _check_compact(st, hq, compact, tp)
+    elif want_compact:
         compact = alloc_compact(st, hq, tp)
     if scan_out is not None:
         if q2kv is not None:
@@ -280,6 +282,24 @@ def alloc_compact(st: IndexState, hq: int, tp: Optional[int] = None) -> CompactR
         tile_parents=tp, tile_rows=tp * st.bf)
 
 
+def compact_fits(st: IndexState, hq: int, c: CompactResult, tp: int) -> bool:
+    """Whether `c` can take what a search of `st` by `hq` heads in tiles of `tp` parents writes.  The tile size
+    is part of that: two indexes of equal capacity need not have the same."""
+    return (c.tile_parents == tp and c.tile_rows == tp * st.bf and c.idx.device == st.children.device
+            and c.idx.shape == c.score.shape == (hq, st.cap_children) and c.count.shape == (hq, n_tiles(st, tp)))
+
+
+def _check_compact(st: IndexState, hq: int, c: CompactResult, tp: int):
+    if not compact_fits(st, hq, c, tp):
+        raise ValueError(f"compact buffers of {tuple(c.idx.shape)} slots and {tuple(c.count.shape)} tiles of {c.tile_parents} "
+                         f"parents do not fit a search of this index by {hq} heads in tiles of {tp}")
+
+
+def compact_for(st: IndexState, hq: int, have: Optional[CompactResult]) -> CompactResult:
+    """`have` where a search of `st` by `hq` heads can reuse it, else new buffers."""
+    return have if have is not None and compact_fits(st, hq, have, tile_parents(st)) else alloc_compact(st, hq)
+
+
 @lru_cache(maxsize=256)
 def _default_splits(hq: int, tiles: int) -> int:   # a pure function of the two numbers
     return int(L.load().hira_attn_default_splits(hq, tiles))
@@ -319,6 +339,7 @@ def sparse_attn(st: IndexState, q, scaling, compact: CompactResult, *, q2kv=None
     last dimension has to be contiguous."""
     lib = L.load()
     hq = q.shape[0]
+    _check_compact(st, hq, compact, compact.tile_parents)
     n_splits = n_splits or attn_splits(st, hq, compact.tile_parents)
     dev = st.device
     if workspace is None:
@@ -432,6 +453,7 @@ def decode_attention(st: IndexState, q: torch.Tensor, sm_scale: float, tau: torc
     dtype the threshold is found on the way, into `tau`."""
     lib = L.load()
     hq = q.shape[0]
+    _check_compact(st, hq, compact, compact.tile_parents)
     n_queued, qstride = 0, 0
     if queued_k is not None and queued_k.shape[-2] > 0:
         n_queued, qstride = _queue_layout(st, queued_k, queued_v)
@@ -458,6 +480,7 @@ def decode_attention(st: IndexState, q: torch.Tensor, sm_scale: float, tau: torc
 def kth_score(st: IndexState, compact: CompactResult, k: torch.Tensor, out=None):
     lib = L.load()
     hq = compact.idx.shape[0]
+    _check_compact(st, hq, compact, compact.tile_parents)
     if out is None:
         out = torch.empty((hq,), dtype=torch.float32, device=st.device)
     rc = lib.hira_kth_score(st.struct, hq, compact.tile_parents, L.ptr(compact.score), L.ptr(compact.count),

@@ -114,9 +114,7 @@ class CUDASearcher(BaseSearcher):
                        scaling: Optional[torch.Tensor] = None, stats: Optional[torch.Tensor] = None) -> S.CompactResult:
         st, q, tau, scaling, q2kv, max_group, qnorm = self._prepare(query, threshold, indexer, q_head_to_kv, scaling)
         hq = q.shape[0]
-        c = self._compact
-        if c is None or c.idx.device != st.device or tuple(c.idx.shape) != (hq, st.cap_children):
-            c = self._compact = S.alloc_compact(st, hq)
+        c = self._compact = S.compact_for(st, hq, self._compact)
         S.search(st, q, tau, scaling=scaling, qnorm=qnorm, q2kv=q2kv, max_group=max_group, flags=self.flags,
                  compact=c, stats=stats)
         return c

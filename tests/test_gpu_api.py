@@ -464,3 +464,24 @@ def test_decode_step_from_host_buffers_equals_the_separate_calls(levels, fused):
     step(q, out_host, threshold=tau2)
     step.synchronize()
     assert torch.equal(got, out_host)
+
+
+def test_one_searcher_on_indexes_of_different_tilings():
+    """The searcher's buffers follow the index it is given: same heads, branching and capacity, another tile size."""
+    from hira_b200 import index_state as S
+    from hira_b200.cache import CacheOutput
+    h, hq, bf = 8, 16, 32
+    one = CUDASearcher(bf)
+    tiles = set()
+    for d, dtype in ((128, torch.bfloat16), (64, torch.bfloat16), (128, torch.bfloat16)):
+        ix = CUDAIndexer(3, 1, bf).build(_keys(h, 9216, d, 21, dtype), _keys(h, 9216, d, 22, dtype))
+        tiles.add((ix.state.cap_children, S.tile_parents(ix.state)))
+        empty = torch.empty((1, h, 0, d), dtype=dtype, device="cuda")
+        q, tau = _query(hq, d, 23), torch.full((hq,), 0.1, device="cuda")
+        outs, lists = [], []
+        for s in (one, CUDASearcher(bf)):
+            outs.append(hira_decode_attention(q, CacheOutput(empty, empty, None, None, ix, s), threshold=tau))
+            lists.append(s.search_compact(q, tau, ix).to_lists())
+        assert torch.equal(*outs)
+        assert all(torch.equal(x, y) for a, b in zip(*lists) for x, y in zip(a, b))
+    assert len({c for c, _ in tiles}) == 1 and len(tiles) == 2
