@@ -108,8 +108,10 @@ class HiraCacheLayer(CacheLayerMixin):
         n = key_states.shape[-2]
         if (self.queued_len == 0 and n >= self.update_every and key_states.dtype == self.dtype
                 and value_states.dtype == self.vdtype and key_states.device == self.device == value_states.device
-                and key_states.shape[:2] == value_states.shape[:2] == self._queue_k.shape[:2]):
-            # nothing waits and a flush is due: straight into the index, without a copy through the queue
+                and key_states.shape == (self.B, self.H_kv, n, self.dim)
+                and value_states.shape == (self.B, self.H_kv, n, self.vdim)):
+            # nothing waits and a flush is due: straight into the index, without a copy through the queue; what
+            # the queue would not take as it is still goes there, to be broadcast or refused
             self.indexer.update(key_states, value_states)
             self.indexed_len += n
         else:

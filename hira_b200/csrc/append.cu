@@ -467,6 +467,16 @@ extern "C" size_t hira_append_workspace_bytes(const hira_index_t* ix, int32_t n_
     return (size_t)ix->n_heads * n_new * (append_parts(ix) + 1) * sizeof(BestRec);
 }
 
+// the kernels read keys and values in 16-byte pieces
+static int check_rows(const char* who, const hira_index_t* ix, const void* new_k, const void* new_v, int64_t k_head_stride,
+                      int64_t v_head_stride) {
+    const int64_t ks = k_head_stride * (int64_t)elem_size(ix->dtype), vs = new_v ? v_head_stride * (int64_t)elem_size(ix->vdtype) : 0;
+    const uint64_t bits = (uint64_t)(uintptr_t)new_k | (uint64_t)(uintptr_t)new_v | (uint64_t)(ix->n_heads > 1 ? ks | vs : 0);
+    HIRA_CHECK_ARG((bits & 15) == 0, HIRA_ERR_ARG,
+                   "%s: new keys and values must start on 16-byte boundaries for every head", who);
+    return HIRA_OK;
+}
+
 extern "C" int hira_append(const hira_index_t* ix, const void* new_k, const void* new_v, int32_t n_new,
                            int64_t k_head_stride, int64_t v_head_stride, int32_t token_base,
                            int32_t* status, void* workspace, size_t workspace_bytes, void* stream) {
@@ -479,6 +489,8 @@ extern "C" int hira_append(const hira_index_t* ix, const void* new_k, const void
     HIRA_CHECK_ARG(ix->parent_sqnorm && (ix->depth == 2 || ix->gp_sqnorm), HIRA_ERR_ARG,
                    "hira_append: the index needs its parent_sqnorm / gp_sqnorm caches");
     if (n_new == 0) return HIRA_OK;
+    rc = check_rows("hira_append", ix, new_k, new_v, k_head_stride, v_head_stride);
+    if (rc != HIRA_OK) return rc;
     AppendParams P;
     P.ix = *ix; P.new_k = new_k; P.new_v = new_v; P.n_new = n_new;
     P.k_head_stride = k_head_stride; P.v_head_stride = v_head_stride;
@@ -509,6 +521,8 @@ extern "C" int hira_append_scanned(const hira_index_t* ix, const void* new_k, co
                    "hira_append_scanned: values must be given iff the index stores values");
     HIRA_CHECK_ARG(ix->parent_sqnorm && (ix->depth == 2 || ix->gp_sqnorm), HIRA_ERR_ARG,
                    "hira_append_scanned: the index needs its parent_sqnorm / gp_sqnorm caches");
+    rc = check_rows("hira_append_scanned", ix, new_k, new_v, k_head_stride, v_head_stride);
+    if (rc != HIRA_OK) return rc;
     AppendParams P;
     P.ix = *ix; P.new_k = new_k; P.new_v = new_v; P.n_new = 1;
     P.k_head_stride = k_head_stride; P.v_head_stride = v_head_stride;

@@ -16,6 +16,11 @@ import torch
 from . import _lib as L
 
 
+def aligned(t: torch.Tensor) -> torch.Tensor:
+    """`t`, or a copy of it where it does not start on a 16-byte boundary: the kernels load rows in 16-byte pieces."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class IndexState:
     def __init__(self, *, n_heads: int, dim: int, vdim: int, bf: int, depth: int, cap_parents: int,
                  dtype: torch.dtype, vdtype: Optional[torch.dtype], device, with_values: bool = True,
@@ -373,14 +378,20 @@ def merge_partials(part_o, part_ml, out=None, out_ml=None):
     return out
 
 
+def _check_rows(t: torch.Tensor, h: int, m: int, width: int, dtype: torch.dtype):
+    if t.shape != (h, m, width):
+        raise ValueError(f"expected ({h}, {m}, {width}) rows, got {tuple(t.shape)}")
+    assert t.is_contiguous() and t.dtype == dtype
+
+
 def append(st: IndexState, new_k: torch.Tensor, new_v: Optional[torch.Tensor], token_base: int = -1,
            use_workspace: bool = True):
-    """new_k (n_heads, M, D), new_v (n_heads, M, V) contiguous, index dtypes."""
+    """new_k (n_heads, M, D), new_v (n_heads, M, V) contiguous, index dtypes, on 16-byte boundaries."""
     lib = L.load()
-    assert new_k.is_contiguous() and new_k.dtype == st.dtype
     m = new_k.shape[1]
+    _check_rows(new_k, st.n_heads, m, st.dim, st.dtype)
     if new_v is not None:
-        assert new_v.is_contiguous() and new_v.dtype == st.vdtype
+        _check_rows(new_v, st.n_heads, m, st.vdim, st.vdtype)
     ws, nbytes = None, 0
     if use_workspace:
         sizes = st._append_bytes     # depends on the heads, the capacity and m only
@@ -407,9 +418,9 @@ def append_scanned(st: IndexState, new_k: torch.Tensor, new_v: Optional[torch.Te
     """One key per head, new_k (n_heads, 1, D) / new_v (n_heads, 1, V) in the index dtypes, whose
     nearest parent the preceding `search(..., scan_key=new_k[:, 0], scan_out=scan)` found."""
     lib = L.load()
-    assert new_k.dtype == st.dtype and new_k.shape[1] == 1 and new_k.stride(-1) == 1
+    assert new_k.dtype == st.dtype and new_k.shape == (st.n_heads, 1, st.dim) and new_k.stride(-1) == 1
     if new_v is not None:
-        assert new_v.dtype == st.vdtype and new_v.stride(-1) == 1
+        assert new_v.dtype == st.vdtype and new_v.shape == (st.n_heads, 1, st.vdim) and new_v.stride(-1) == 1
     rc = lib.hira_append_scanned(st.struct, L.ptr(new_k), L.ptr(new_v), new_k.stride(0),
                                  new_v.stride(0) if new_v is not None else 0, token_base, L.ptr(st.status),
                                  L.ptr(scan), L.current_stream(st.device))

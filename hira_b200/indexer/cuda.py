@@ -130,15 +130,15 @@ class CUDAIndexer(BaseIndexer):
         if t.ndim != 4:
             raise ValueError(f"expected a (B, H, L, D) tensor, got {tuple(t.shape)}")
         b, h, l, d = t.shape
-        return t.reshape(b * h, l, d).contiguous()
+        return S.aligned(t.reshape(b * h, l, d).contiguous())
 
     def _rows(self, t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
-        """(B, H, M, D) as contiguous (B*H, M, D) rows of the index's device and `dtype`."""
+        """(B, H, M, D) as contiguous (B*H, M, D) rows of the index's device and `dtype` from a 16-byte boundary."""
         if t.dtype != dtype or t.device != self.state.device or not t.is_contiguous():
             return self._fold(t.to(self.state.device)).to(dtype)
         if t.ndim != 4:
             raise ValueError(f"expected a (B, H, L, D) tensor, got {tuple(t.shape)}")
-        return t.view(-1, t.shape[2], t.shape[3]) if t.shape[0] != 1 else t[0]
+        return S.aligned(t.view(-1, t.shape[2], t.shape[3]) if t.shape[0] != 1 else t[0])
 
     @staticmethod
     def _stratified(h: int, n: int, k: int, g: torch.Generator, device) -> torch.Tensor:
@@ -324,6 +324,8 @@ class CUDAIndexer(BaseIndexer):
         if st.values is not None:
             if new_values is None:
                 raise ValueError("the index stores values: new_values is required")
+            if new_values.shape[3] != st.vdim:
+                raise ValueError(f"new_values are {new_values.shape[3]} wide, the index stores {st.vdim}")
             v = self._rows(new_values, st.vdtype)
         if m == 0:
             return self

@@ -285,7 +285,8 @@ int hira_exchange_merge(const float* local_rows, void* const* peer_bufs,
  * after another in order, so the result is deterministic.
  *
  *   new_k [n_heads][n_new][dim], new_v [n_heads][n_new][vdim]: index dtypes,
- *          head strides in elements
+ *          head strides in elements; every head's rows start on a 16-byte boundary
+ *          (other addresses are refused)
  *   token_base: token position of new key 0 is token_base + used[h][2]
  *          when token_base < 0, else token_base + i
  *   status: device int32, OR-ed with HIRA_STATUS_* on capacity exhaustion

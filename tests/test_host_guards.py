@@ -1,11 +1,13 @@
 """Host-side guards between the Python classes and the kernels, on the CPU: a call whose buffers do not fit what a
 kernel would write or read is refused, or given buffers that do, before anything is launched."""
+import ctypes
 from types import SimpleNamespace
 
 import pytest
 import torch
 
-from hira_b200 import CUDASearcher, hira_decode_attention
+from hira_b200 import CUDAIndexer, CUDASearcher, DeviceMode, HiraCacheLayer, hira_decode_attention
+from hira_b200 import _lib as L
 from hira_b200 import index_state as S
 
 
@@ -48,3 +50,89 @@ def test_one_searcher_serves_indexes_of_different_tilings(monkeypatch):
         tp = S.tile_parents(st)
         assert (c.tile_parents, c.tile_rows) == (tp, tp * st.bf) and c.count.shape == (hq, S.n_tiles(st, tp))
     assert seen[2][2] is seen[4][2] and seen[3][2] is seen[5][2]     # kept while the index stays the same
+
+
+def _indexer(h=4, dim=64, vdim=64, dtype=torch.bfloat16):
+    """An indexer on host memory: its appends are recorded by `_record_appends`."""
+    ix = CUDAIndexer(3, 1, 8, max_context=4096)
+    ix.state = S.IndexState(n_heads=h, dim=dim, vdim=vdim, bf=8, depth=3, cap_parents=512, dtype=dtype, vdtype=dtype, device="cpu")
+    ix.num_heads, ix.dim = h, dim
+    return ix
+
+
+def _record_appends(monkeypatch):
+    seen = []
+
+    def append(st, k, v, *a, **kw):
+        S._check_rows(k, st.n_heads, k.shape[1], st.dim, st.dtype)
+        S._check_rows(v, st.n_heads, k.shape[1], st.vdim, st.vdtype)
+        assert k.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0
+        seen.append((k, v))
+    monkeypatch.setattr(S, "append", append)
+    return seen
+
+
+def _layer(ix, update_every=1):
+    layer = HiraCacheLayer(DeviceMode.CUDA_ONLY, update_every, {}, {})
+    layer.indexer_cls, layer.searcher_cls = lambda **kw: ix, lambda **kw: None
+    ix.build = lambda k, v: ix
+    st = ix.state
+    layer.update(torch.zeros(1, st.n_heads, 3, st.dim, dtype=st.dtype), torch.zeros(1, st.n_heads, 3, st.vdim, dtype=st.dtype))
+    return layer
+
+
+def _off_by(shape, elements, dtype=torch.bfloat16):
+    """A contiguous tensor that starts `elements` behind a 16-byte boundary, as a view into a fused projection does."""
+    n = torch.Size(shape).numel()
+    t = torch.arange(n + elements).to(dtype)[elements:].view(shape)
+    assert t.is_contiguous() and t.data_ptr() % 16 == elements * t.element_size() % 16
+    return t
+
+
+@pytest.mark.parametrize("width", [32, 72, 128])
+def test_values_of_another_width_are_refused(monkeypatch, width):
+    seen = _record_appends(monkeypatch)
+    ix = _indexer()
+    layer = _layer(ix)
+    with pytest.raises(RuntimeError):            # as the queue refuses them
+        layer.update(torch.zeros(1, 4, 1, 64, dtype=torch.bfloat16), torch.zeros(1, 4, 1, width, dtype=torch.bfloat16))
+    with pytest.raises(ValueError, match="wide"):
+        ix.update(torch.zeros(1, 4, 1, 64, dtype=torch.bfloat16), torch.zeros(1, 4, 1, width, dtype=torch.bfloat16))
+    assert not seen
+
+
+def test_what_the_queue_broadcasts_is_still_broadcast(monkeypatch):
+    seen = _record_appends(monkeypatch)
+    layer = _layer(_indexer())
+    k, v = torch.randn(1, 4, 3, 64).bfloat16(), torch.randn(1, 4, 1, 1).bfloat16()
+    layer.update(k, v)
+    assert torch.equal(seen[0][0], k[0]) and torch.equal(seen[0][1], v[0].expand(4, 3, 64)) and layer.get_seq_length() == 6
+
+
+@pytest.mark.parametrize("elements", [0, 1, 4, 7])
+@pytest.mark.parametrize("batch", [1, 2])
+def test_unaligned_keys_and_values_are_copied_to_a_boundary(monkeypatch, elements, batch):
+    seen = _record_appends(monkeypatch)
+    ix = _indexer()
+    k, v = _off_by((batch, 4 // batch, 2, 64), elements), _off_by((batch, 4 // batch, 2, 64), 2 * elements)
+    ix.update(k, v)
+    if batch == 1:
+        _layer(ix, 2).update(k, v)
+    for a, b in seen:
+        assert torch.equal(a, k.view(4, 2, 64)) and torch.equal(b, v.view(4, 2, 64))
+        assert elements or a.data_ptr() == k.data_ptr()      # nothing is copied without need
+    assert len(seen) == 3 - batch
+    assert ix.begin_scanned_update(k[:, :, :1])[0].data_ptr() % 16 == 0
+
+
+def test_append_refuses_unaligned_rows_before_any_launch():
+    lib, st = L.load(), _indexer().state
+    status = torch.zeros(1, dtype=torch.int32)
+    base = torch.zeros(4 * 2 * 64 + 8, dtype=torch.bfloat16).data_ptr()
+    assert base % 16 == 0
+    for k, v, ks, vs in ((base + 2, base, 64, 64), (base, base + 8, 64, 64), (base, base, 68, 64), (base, base, 64, 65)):
+        for rc in (lib.hira_append(st.struct, k, v, 1, ks, vs, -1, status.data_ptr(), None, 0, None),
+                   lib.hira_append_scanned(st.struct, k, v, ks, vs, -1, status.data_ptr(), status.data_ptr(), None)):
+            assert rc == L.HIRA_ERR_ARG and b"16-byte" in lib.hira_last_error()
+    with pytest.raises(ValueError, match="rows"):
+        S.append(st, torch.zeros(4, 1, 64, dtype=torch.bfloat16), torch.zeros(4, 1, 32, dtype=torch.bfloat16))
