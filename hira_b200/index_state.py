@@ -77,6 +77,8 @@ class IndexState:
         self.status = z((1,), dtype=torch.int32, device=dev)
         self._struct = None
         self._append_bytes = {}
+        # streams the arrays are kept alive for: the one they are allocated on, and those of `used_on`
+        self._streams = {L.current_stream(dev)} if dev.type == "cuda" else set()
         self._active_parents = 0
         self.refresh_struct()
 
@@ -117,6 +119,17 @@ class IndexState:
             return
         self._active_parents = n
         self._struct.active_parents = n
+
+    def used_on(self, stream):
+        """Keeps the memory of the arrays from being handed out again before the work enqueued on `stream` when
+        they are dropped is done."""
+        if stream.cuda_stream in self._streams:
+            return
+        self._streams.add(stream.cuda_stream)
+        for name in self.ARRAYS + self.Q8_ARRAYS + ("status",):
+            t = getattr(self, name)
+            if t is not None:
+                t.record_stream(stream)
 
     @property
     def struct(self):
@@ -162,6 +175,7 @@ class IndexState:
                          with_values=self.values is not None, int8_copy=self.int8_copy, cleared=self.device.type != "cuda")
         new.status.copy_(self.status)
         if self.device.type == "cuda":
+            self.used_on(torch.cuda.current_stream(self.device))     # the caller drops the old arrays right away
             old = L.HiraIndexStruct.from_buffer_copy(self._struct)
             for name in self.Q8_ARRAYS:     # also when enable_int8_copy has left them out of the view
                 setattr(old, name, L.ptr(getattr(self, name)))
@@ -399,9 +413,11 @@ def append(st: IndexState, new_k: torch.Tensor, new_v: Optional[torch.Tensor], t
         if nbytes is None:
             nbytes = sizes[m] = int(lib.hira_append_workspace_bytes(st.struct, m))
         if nbytes:
-            ws = getattr(st, "_append_ws", None)
-            if ws is None or ws.numel() < nbytes:
-                ws = st._append_ws = torch.empty((nbytes,), dtype=torch.uint8, device=st.device)
+            ws, home = getattr(st, "_append_ws", (None, 0))
+            stream = L.current_stream(st.device)
+            if ws is None or ws.numel() < nbytes or home != stream:    # scratch of the stream it is used on
+                ws = torch.empty((nbytes,), dtype=torch.uint8, device=st.device)
+                st._append_ws = ws, stream
     rc = lib.hira_append(st.struct, L.ptr(new_k), L.ptr(new_v), m, m * st.dim,
                          m * st.vdim if new_v is not None else 0, token_base, L.ptr(st.status),
                          L.ptr(ws), nbytes, L.current_stream(st.device))

@@ -221,7 +221,8 @@ class CUDAIndexer(BaseIndexer):
         return self
 
     # ---- update -------------------------------------------------------------
-    def _ensure_capacity(self, m: int):
+    def _ensure_capacity(self, m: int, home=None):
+        """`home`: the stream the index lives on, when the current one is a side stream of an update."""
         st = self.state
         need_p = self._parents_bound + m
         need_g = self._gp_bound + m
@@ -241,7 +242,16 @@ class CUDAIndexer(BaseIndexer):
             if need_p <= st.cap_parents:
                 return
             new_cap = max(need_p, st.cap_parents + max(1, st.cap_parents // 2))
-        self.state = st.grown(new_cap)
+        if home is None:
+            self.state = st.grown(new_cap)
+            return
+        # The index moves on the stream it lives on: behind the appends so far and behind the attention that may
+        # still read the old arrays, whose memory is that stream's to hand out again, as is that of the new ones.
+        side = torch.cuda.current_stream(st.device)
+        home.wait_stream(side)
+        with torch.cuda.stream(home):
+            self.state = st.grown(new_cap)
+        side.wait_stream(home)
 
     # ---- updates beside the attention, on a second stream ---------------------
     def searched_event(self) -> int:
@@ -306,11 +316,15 @@ class CUDAIndexer(BaseIndexer):
                     if t is not None and t.is_cuda:
                         t.record_stream(stream)
                 with torch.cuda.stream(stream):
-                    self.update(new_keys, new_values, scanned=scanned)
+                    self._update(new_keys, new_values, scanned, home=cur)
                     done = torch.cuda.Event()
                     done.record(stream)
                 self._pending_append = done
                 return self
+        return self._update(new_keys, new_values, scanned)
+
+    def _update(self, new_keys, new_values, scanned: bool, home=None):
+        """`update` on the current stream; `home`: see `_ensure_capacity`."""
         self.wait_pending_update()
         assert new_values is None or new_keys.shape[:3] == new_values.shape[:3]
         if new_keys.ndim != 4:
@@ -329,7 +343,11 @@ class CUDAIndexer(BaseIndexer):
             v = self._rows(new_values, st.vdtype)
         if m == 0:
             return self
-        self._ensure_capacity(m)
+        self._ensure_capacity(m, home)
+        if home is not None:     # what the index owns may be dropped while the append still runs
+            self.state.used_on(torch.cuda.current_stream(self.state.device))
+            if self._scan_slots is not None:
+                self._scan_slots.record_stream(torch.cuda.current_stream(self.state.device))
         if scanned:
             if m != 1 or not self._scan_pending:
                 raise ValueError("update(scanned=True) needs one key per head and a search that scanned for it")

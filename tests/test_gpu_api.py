@@ -485,3 +485,48 @@ def test_one_searcher_on_indexes_of_different_tilings():
         assert torch.equal(*outs)
         assert all(torch.equal(x, y) for a, b in zip(*lists) for x, y in zip(a, b))
     assert len({c for c, _ in tiles}) == 1 and len(tiles) == 2
+
+
+def _pool_stream(t):
+    """The stream whose allocator pool the memory of `t` belongs to."""
+    for seg in torch.cuda.memory_snapshot():
+        if seg["address"] <= t.data_ptr() < seg["address"] + seg["total_size"]:
+            return seg["stream"]
+    raise AssertionError("not from the caching allocator")
+
+
+def test_growth_during_a_side_stream_update_stays_in_the_main_pool():
+    h, n, d, bf = 4, 4096, 64, 8
+    keys, vals = _keys(h, n, d, 31), _keys(h, n, d, 32)
+    a, b = (CUDAIndexer(3, 1, bf, seed=5).build(keys, vals) for _ in range(2))     # no room reserved: the first append grows
+    more_k, more_v = _keys(h, 12, d, 33), _keys(h, 12, d, 34)
+    torch.cuda.synchronize()
+    side, before = torch.cuda.Stream(), b.state
+    for i in range(12):
+        a.update(more_k[:, :, i:i + 1], more_v[:, :, i:i + 1])
+        b.update(more_k[:, :, i:i + 1], more_v[:, :, i:i + 1], stream=side)
+    a.check_status(), b.check_status()
+    assert b.state is not before
+    for name in a.state.ARRAYS:
+        x, y = getattr(a.state, name), getattr(b.state, name)
+        assert x is None and y is None or torch.equal(x, y), name
+        if y is not None:
+            assert _pool_stream(y) == torch.cuda.current_stream().cuda_stream, name
+
+
+def test_arrays_dropped_during_a_side_stream_update_are_not_handed_out():
+    h, n, d, bf = 4, 16384, 64, 16
+    keys, vals = _keys(h, n, d, 35), _keys(h, n, d, 36)
+    ix = CUDAIndexer(3, 1, bf, max_context=n + 8).build(keys, vals)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)        # some 50 ms
+    k = keys[:, :, :1].contiguous()
+    ix.update(k, k, stream=side)
+    ptr, like = ix.children.data_ptr(), torch.empty_like(ix.children, device="meta")
+    del ix
+    again = [torch.empty(like.shape, dtype=like.dtype, device="cuda") for _ in range(2)]
+    busy = not side.query()
+    assert all(t.data_ptr() != ptr for t in again) or not busy
+    side.synchronize()

@@ -136,3 +136,50 @@ def test_append_refuses_unaligned_rows_before_any_launch():
             assert rc == L.HIRA_ERR_ARG and b"16-byte" in lib.hira_last_error()
     with pytest.raises(ValueError, match="rows"):
         S.append(st, torch.zeros(4, 1, 64, dtype=torch.bfloat16), torch.zeros(4, 1, 32, dtype=torch.bfloat16))
+
+
+class _FakeStream:
+    cuda_stream = 0
+
+    def __init__(self, name, log):
+        self.name, self.log = name, log
+
+    def wait_stream(self, other):
+        self.log.append((self.name, "waits for", other.name))
+
+    def wait_event(self, event):
+        self.log.append((self.name, "waits for", "event"))
+
+
+def test_growth_of_a_side_stream_update_runs_where_the_index_lives(monkeypatch):
+    """The old arrays are read, and the new ones allocated, on the stream whose memory they are."""
+    log = []
+    main, side = _FakeStream("main", log), _FakeStream("side", log)
+    active = [main]
+
+    class _On:
+        def __init__(self, s):
+            self.s = s
+
+        def __enter__(self):
+            active.append(self.s)
+
+        def __exit__(self, *a):
+            active.pop()
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: active[-1])
+    monkeypatch.setattr(torch.cuda, "stream", _On)
+    monkeypatch.setattr(torch.cuda, "Event", lambda: SimpleNamespace(record=lambda s: log.append((s.name, "record"))))
+    grown = S.IndexState.grown
+    monkeypatch.setattr(S.IndexState, "grown", lambda st, n: log.append((active[-1].name, "grows")) or grown(st, n))
+    monkeypatch.setattr(S.IndexState, "used_on", lambda st, s: log.append((s.name, "uses", st.cap_parents)), raising=False)
+    monkeypatch.setattr(S, "append", lambda st, k, v: log.append((active[-1].name, "appends")))
+    ix = _indexer()
+    ix._parents_bound, ix._gp_bound = ix.state.cap_parents, ix.state.cap_gp
+    ix.state.used[:, 0], ix.state.used[:, 1] = ix._parents_bound, ix._gp_bound
+    row = torch.zeros(1, 4, 1, 64, dtype=torch.bfloat16)
+    ix.update(row, row, stream=side)
+    assert log == [("side", "waits for", "main"), ("main", "waits for", "side"), ("main", "grows"), ("side", "waits for", "main"),
+                   ("side", "uses", 768), ("side", "appends"), ("side", "record")]
+    log.clear()
+    ix.update(row, row)
+    assert log == [("main", "waits for", "event"), ("main", "appends")]
