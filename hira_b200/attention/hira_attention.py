@@ -104,8 +104,7 @@ def hira_decode_attention(query: torch.Tensor, cache_output, *, scaling: Optiona
         stride = S.queue_stride(qk) if qk.dtype == st.dtype and qk.device == st.device else None
         if stride is None or qv.dtype != st.vdtype or qv.device != st.device or S.queue_stride(qv) != stride:
             # not the filled part of two like queue buffers: a dense copy
-            queued_k = qk.reshape(-1, qk.shape[-2], qk.shape[-1]).to(st.dtype).contiguous()
-            queued_v = qv.reshape(-1, qv.shape[-2], qv.shape[-1]).to(st.vdtype).contiguous()
+            queued_k, queued_v = S.dense_rows(qk, st.dtype, st.device), S.dense_rows(qv, st.vdtype, st.device)
     n_splits = S.attn_splits(st, n_q, compact.tile_parents)
     ws = getattr(srch, "_attn_ws", None)
     need = n_q * n_splits * (st.vdim + 2)

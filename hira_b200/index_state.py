@@ -332,14 +332,22 @@ def attn_splits(st: IndexState, hq: int, tp: Optional[int] = None) -> int:
 
 def queue_stride(t: torch.Tensor) -> Optional[int]:
     """Elements between the heads of a (B, H, n, D) or (H, n, D) queue whose rows lie one behind another from
-    a 16-byte boundary -- a whole tensor or the filled part of a queue buffer --, None for any other layout."""
-    d, strides = t.shape[-1], t.stride()
-    hs = strides[-3]
-    if strides[-1] != 1 or strides[-2] != d or hs < t.shape[-2] * d or t.data_ptr() % 16 or hs * t.element_size() % 16:
+    a 16-byte boundary -- a whole tensor or the filled part of a queue buffer --, None for any other layout.
+    A stride along a dimension of one says nothing and is not looked at."""
+    (h, n, d), (hs, ns, ds) = t.shape[-3:], t.stride()[-3:]
+    b, bs = (t.shape[0], t.stride(0)) if t.ndim == 4 else (1, 0)
+    if h == 1:                       # the heads to step over are the batch
+        h, hs, b = b, bs, 1
+    if h == 1:
+        hs = n * d
+    if ds != 1 or (n > 1 and ns != d) or hs < n * d or t.data_ptr() % 16 or hs * t.element_size() % 16:
         return None
-    if t.ndim == 4 and t.shape[0] > 1 and strides[0] != t.shape[1] * hs:
-        return None
-    return hs
+    return hs if b == 1 or bs == h * hs else None
+
+
+def dense_rows(t: torch.Tensor, dtype: torch.dtype, device) -> torch.Tensor:
+    """A (..., n, D) queue as (H, n, D) rows that `queue_stride` accepts, copied where it does not as it is."""
+    return aligned(t.reshape(-1, t.shape[-2], t.shape[-1]).to(device=device, dtype=dtype).contiguous())
 
 
 def _queue_layout(st: IndexState, queued_k: torch.Tensor, queued_v: torch.Tensor):
@@ -348,7 +356,8 @@ def _queue_layout(st: IndexState, queued_k: torch.Tensor, queued_v: torch.Tensor
     if st.vdim != st.dim:
         raise ValueError("queued keys/values with vdim != dim are not supported")
     stride = queue_stride(queued_k)
-    assert stride is not None and stride == queue_stride(queued_v)
+    if stride is None or stride != queue_stride(queued_v):
+        raise ValueError("queued keys and values must be rows one behind another from a 16-byte boundary, with one head stride")
     return queued_k.shape[-2], stride
 
 

@@ -183,3 +183,44 @@ def test_growth_of_a_side_stream_update_runs_where_the_index_lives(monkeypatch):
     log.clear()
     ix.update(row, row)
     assert log == [("main", "waits for", "event"), ("main", "appends")]
+
+
+def _odd_queues():
+    """Queues that are dense, or become so by a copy, in layouts a caller can come by; (keys, values) of 4 heads."""
+    def whole(n, b=1):
+        return torch.randn(b, 4 // b, n, 64).bfloat16()
+    yield "whole", whole(3), whole(3)
+    yield "batch", whole(3, 2), whole(3, 2)
+    yield "filled part", whole(8, 2)[:, :, :3], whole(8, 2)[:, :, :3]
+    yield "another head stride", whole(8)[:, :, :3], whole(5)[:, :, :3]
+    yield "unaligned", _off_by((1, 4, 3, 64), 1), _off_by((1, 4, 3, 64), 3)
+    yield "unaligned values", whole(3), _off_by((1, 4, 3, 64), 4)
+    yield "one row, transposed", torch.randn(1, 1, 4, 64).bfloat16().transpose(1, 2), torch.randn(1, 1, 4, 64).bfloat16().transpose(1, 2)
+    yield "one head a batch item", whole(3, 4), torch.randn(3, 4, 1, 64).bfloat16().permute(1, 2, 0, 3)
+    yield "strides of ones", whole(1).as_strided((1, 4, 1, 64), (7, 64, 9, 1)), whole(1).as_strided((1, 4, 1, 64), (1, 64, 1, 1))
+    yield "broadcast", whole(1).expand(1, 4, 3, 64), whole(3)
+    yield "floats", whole(3).float(), whole(3).float()
+
+
+@pytest.mark.parametrize("what,qk,qv", [pytest.param(*c, id=c[0]) for c in _odd_queues()])
+def test_queues_of_any_layout_reach_the_attention(monkeypatch, what, qk, qv):
+    seen = []
+    monkeypatch.setattr(S, "decode_attention", lambda *a, queued_k, queued_v, **kw: seen.append((queued_k, queued_v)))
+    ix = _indexer()
+    out = SimpleNamespace(indexer=SimpleNamespace(state=ix.state), searcher=CUDASearcher(), queued_keys=qk, queued_values=qv)
+    hira_decode_attention(torch.zeros(1, 8, 1, 64), out, threshold=torch.zeros(8))
+    n, stride = S._queue_layout(ix.state, *seen[0])
+    assert n == qk.shape[-2]
+    for got, want in zip(seen[0], (qk, qv)):
+        assert got.data_ptr() % 16 == 0
+        assert torch.equal(torch.as_strided(got, (4, n, 64), (stride, 64, 1)), want.reshape(4, n, 64).bfloat16())
+    if what in ("whole", "batch", "filled part", "one row, transposed"):
+        assert seen[0][0] is qk and seen[0][1] is qv       # read in place
+
+
+def test_dense_three_dimensional_queues_are_taken():
+    st = _indexer().state
+    row = torch.randn(1, 4, 64).bfloat16().transpose(0, 1)      # (H, 1, D), contiguous whatever its row stride
+    assert row.is_contiguous() and S._queue_layout(st, row, row) == (1, 64)
+    with pytest.raises(ValueError, match="16-byte"):
+        S._queue_layout(st, _off_by((4, 3, 64), 1), _off_by((4, 3, 64), 1))
