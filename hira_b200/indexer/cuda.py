@@ -138,7 +138,7 @@ class CUDAIndexer(BaseIndexer):
             return self._fold(t.to(self.state.device)).to(dtype)
         if t.ndim != 4:
             raise ValueError(f"expected a (B, H, L, D) tensor, got {tuple(t.shape)}")
-        return S.aligned(t.view(-1, t.shape[2], t.shape[3]) if t.shape[0] != 1 else t[0])
+        return S.aligned(t[0] if t.shape[0] == 1 else t.view(self.num_heads, t.shape[2], t.shape[3]))
 
     @staticmethod
     def _stratified(h: int, n: int, k: int, g: torch.Generator, device) -> torch.Tensor:

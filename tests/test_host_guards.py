@@ -224,3 +224,11 @@ def test_dense_three_dimensional_queues_are_taken():
     assert row.is_contiguous() and S._queue_layout(st, row, row) == (1, 64)
     with pytest.raises(ValueError, match="16-byte"):
         S._queue_layout(st, _off_by((4, 3, 64), 1), _off_by((4, 3, 64), 1))
+
+
+@pytest.mark.parametrize("batch", [1, 2])
+def test_an_update_without_keys_changes_nothing(monkeypatch, batch):
+    seen = _record_appends(monkeypatch)
+    ix = _indexer()
+    none = torch.zeros(batch, 4 // batch, 0, 64, dtype=torch.bfloat16)
+    assert ix.update(none, none) is ix and not seen and ix._appended == 0
