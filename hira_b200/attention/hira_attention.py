@@ -33,9 +33,9 @@ def _samples_for(indexer, sample_size: int) -> torch.Tensor:
     """(H_kv, S, D) key rows drawn once per built index from its filled slots."""
     st = indexer.state
     cached = getattr(indexer, "_tau_samples", None)
-    if cached is not None and cached[0] is st and cached[1].shape[1] == min(sample_size, 4096):
+    s = max(1, min(sample_size, 4096))
+    if cached is not None and cached[0] is st and cached[1].shape[1] == s:
         return cached[1]
-    s = min(sample_size, 4096)
     g = torch.Generator(device=st.device)
     g.manual_seed(getattr(indexer, "seed", 0) + 17)
     filled = st.slot2token >= 0                                   # (H, capC)

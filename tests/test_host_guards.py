@@ -232,3 +232,15 @@ def test_an_update_without_keys_changes_nothing(monkeypatch, batch):
     ix = _indexer()
     none = torch.zeros(batch, 4 // batch, 0, 64, dtype=torch.bfloat16)
     assert ix.update(none, none) is ix and not seen and ix._appended == 0
+
+
+@pytest.mark.parametrize("sample_size,want", [(-3, 1), (0, 1), (1, 1), (40, 40), (64, 64), (1000, 64)])
+def test_threshold_samples_are_at_least_one_and_at_most_the_keys(sample_size, want):
+    from hira_b200.attention.hira_attention import _samples_for
+    for built in (0, 64):                       # loaded from arrays (the keys are counted), or built from 64 of them
+        ix = SimpleNamespace(state=_state(64, n_heads=4, bf=8, cap_parents=16, dtype=torch.float32), _built_keys=built)
+        ix.state.slot2token[:, :64] = torch.arange(64)
+        ix.state.children[:, :64] = 1.0
+        rows = _samples_for(ix, sample_size)
+        assert rows.shape == (4, want, 64) and bool((rows == 1.0).all())
+        assert _samples_for(ix, sample_size).shape == rows.shape
