@@ -454,8 +454,8 @@ using namespace hira;
 static int append_parts(const hira_index_t* ix) {
     // two CTAs per SM, all resident at once, where that leaves enough slices; with many heads several waves of
     // shorter ones; slices of at least 128 parents
-    int parts = 2 * 148 / ix->n_heads - 1;
-    if (parts < 9) parts = (8 * 148 + ix->n_heads - 1) / ix->n_heads < 9 ? (8 * 148 + ix->n_heads - 1) / ix->n_heads : 9;
+    int parts = 2 * SM_COUNT / ix->n_heads - 1;
+    if (parts < 9) parts = (8 * SM_COUNT + ix->n_heads - 1) / ix->n_heads < 9 ? (8 * SM_COUNT + ix->n_heads - 1) / ix->n_heads : 9;
     const int max_parts = ix->cap_parents / 128;
     if (parts > max_parts) parts = max_parts;
     if (parts > 64) parts = 64;

@@ -406,7 +406,7 @@ extern "C" int hira_attn_default_splits(int32_t n_qheads, int32_t n_tiles) {
     // little over a whole number of waves pays for a nearly empty last one.  Measured: 64 query
     // heads 41 -> 34 us against the former 16 CTAs/SM target, 512 query heads unchanged.
     const int factor = 5;   // CTAs per SM aimed for
-    int s = (factor * 148) / n_qheads;
+    int s = (factor * SM_COUNT) / n_qheads;
     if (s > n_tiles) s = n_tiles;
     if (s > 64) s = 64;
     return s < 1 ? 1 : s;

@@ -51,6 +51,7 @@ __device__ __forceinline__ void memcpy_chunk(RawChunk<T>& raw, const T* src) {
 // on their way before the chain needs them.  Eight 16-byte pieces are loaded ahead (before: one element per
 // load; 8 x 1,024 bf16 centres of 128 channels: 18.5 -> 3.1 us).
 constexpr int SQ_THREADS = 64;
+constexpr int MEMBER_LISTS = 2;   // words behind the member counts, see member_starts_kernel
 template <typename T>
 __global__ void __launch_bounds__(SQ_THREADS)
 sqnorm_seq_kernel(const T* __restrict__ rows, long long n_rows, int dim, float* __restrict__ out,
@@ -81,7 +82,11 @@ sqnorm_seq_kernel(const T* __restrict__ rows, long long n_rows, int dim, float* 
         }
     }
     out[i] = acc;
-    if (zero) zero[i] = 0;   // the centre's member count, for the assignment that follows
+    if (zero) {   // the centre's member count and, behind the counts, the work lists' lengths, for the assignment that follows
+        zero[i] = 0;
+        if (i == 0)
+            for (int u = 0; u < MEMBER_LISTS; ++u) zero[n_rows + u] = 0;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -282,40 +287,59 @@ __global__ void gather_centres_kernel(const T* __restrict__ points, long long p_
 // Members of every centre in (distance, point) order.
 //
 // The points of a head are counted per centre, the counts scanned, the points dropped into their centre's
-// range in arrival order and each range sorted by itself: a range is bf points on average, so nearly all of
-// them are sorted by one warp in registers.  The sort key is (distance bits, point), which no two members
-// share, so the result does not depend on the arrival order.  (A device-wide radix sort of (centre, distance)
-// before: 5 or 6 passes of about 9 us whatever the size; 8 x 32,768 points in
-// 1,024 centres each 65 -> 30 us, 8 x 4,096 points in 64 73 -> 22 us with all of the kernels around it.)
+// range in arrival order and each range sorted by itself.  The sort key is (distance bits, point), which no two
+// members share, so the result does not depend on the arrival order.  A range is bf points on average and most are
+// sorted by one warp in registers, but any of them can be anything up to all the points of a head (hubs, padding
+// rows, constant keys): ranges of more than SORT_WARP members go to a work list in pieces of SORT_CTA, a piece is
+// sorted by one CTA, and ranges of several pieces are merged MERGE_WAYS runs at a time by the whole GPU.
+// (A device-wide radix sort of (centre, distance) before: 5 or 6 passes of about 9 us whatever the size; 8 x 32,768
+// points in 1,024 centres each 65 -> 30 us, 8 x 4,096 points in 64 73 -> 22 us with all of the kernels around it.)
 // ---------------------------------------------------------------------------
+constexpr int SORT_THREADS = 256, SORT_RANGES = SORT_THREADS / 32, SORT_WARP = 128, SORT_CTA = 4096;
+constexpr int SORT_PIECE_CTAS = 2 * SM_COUNT;   // CTAs of the sort that serve the work list
+constexpr int MERGE_WAYS = 16, MERGE_UNIT = 1024, MERGE_FLIGHT = 5;
+struct MemberLists {       // pieces as range << 32 | piece: of ranges above SORT_WARP, of ranges above SORT_CTA
+    uint64_t *pieces, *merges;
+    int32_t* len;          // [MEMBER_LISTS]: entries of the two
+};
+static size_t pieces_bound(size_t total) { return total / SORT_WARP + total / SORT_CTA + 1; }   // ceil(m / SORT_CTA) for every m > SORT_WARP
+static size_t merges_bound(size_t total) { return 2 * (total / SORT_CTA) + 1; }                 // the same for every m > SORT_CTA
 
 // An assignment outside [0, k) -- the tensor-core kernel writes -1 for the points of a CTA whose
 // bounded barrier wait ran out -- must not reach the segment arithmetic below: the point goes to
 // centre 0 at distance 0 (so that every later index stays in range) and the caller is told through
 // the status word.
 // `placed` (balanced rounds): points that already have a slot belong to no centre any more (arrival -1).
-__global__ void count_members_kernel(int32_t* __restrict__ idx, float* __restrict__ d2, int n, int k, long long total,
-                                     const int32_t* __restrict__ placed, int32_t* __restrict__ cnt,
-                                     int32_t* __restrict__ arrival, int32_t* __restrict__ status) {
+// The lanes of a warp that chose the same centre count it together: a centre that draws every point of a head
+// would otherwise be one chain of n atomics.
+__global__ void __launch_bounds__(256)
+count_members_kernel(int32_t* __restrict__ idx, float* __restrict__ d2, int n, int k, long long total,
+                     const int32_t* __restrict__ placed, int32_t* __restrict__ cnt, int32_t* __restrict__ arrival,
+                     int32_t* __restrict__ status) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    if (placed && placed[i] >= 0) {
-        arrival[i] = -1;
-        return;
+    const bool counts = i < total && !(placed && placed[i] >= 0);
+    int seg = -1;
+    if (counts) {
+        int c = idx[i];
+        if (c < 0 || c >= k || !(d2[i] >= 0.f)) {
+            if (status) atomicOr(status, HIRA_STATUS_ASSIGN_FAILED);
+            idx[i] = c = 0;
+            d2[i] = 0.f;
+        }
+        seg = (int)(i / n) * k + c;
     }
-    int c = idx[i];
-    if (c < 0 || c >= k || !(d2[i] >= 0.f)) {
-        if (status) atomicOr(status, HIRA_STATUS_ASSIGN_FAILED);
-        idx[i] = c = 0;
-        d2[i] = 0.f;
-    }
-    arrival[i] = atomicAdd(cnt + (i / n) * k + c, 1);
+    const unsigned same = __match_any_sync(0xffffffffu, seg);
+    const int wl = threadIdx.x & 31, leader = __ffs(same) - 1;
+    int at = 0;
+    if (counts && wl == leader) at = atomicAdd(cnt + seg, __popc(same));
+    at = __shfl_sync(0xffffffffu, at, leader);
+    if (i < total) arrival[i] = counts ? at + __popc(same & ((1u << wl) - 1u)) : -1;
 }
 
-// start[h][c] = h n + members of the centres before c
+// start[h][c] = h n + members of the centres before c; and the work lists
 constexpr int SCAN_ITEMS = 4;
 __global__ void __launch_bounds__(1024)
-member_starts_kernel(const int32_t* __restrict__ cnt, int n, int k, int32_t* __restrict__ start) {
+member_starts_kernel(const int32_t* __restrict__ cnt, int n, int k, int32_t* __restrict__ start, const MemberLists lists) {
     typedef cub::BlockScan<int, 1024> Scan;
     __shared__ typename Scan::TempStorage tmp;
     const int h = blockIdx.x;
@@ -324,7 +348,19 @@ member_starts_kernel(const int32_t* __restrict__ cnt, int n, int k, int32_t* __r
         int v[SCAN_ITEMS], total;
         const int c = c0 + threadIdx.x * SCAN_ITEMS;
 #pragma unroll
-        for (int u = 0; u < SCAN_ITEMS; ++u) v[u] = c + u < k ? cnt[(size_t)h * k + c + u] : 0;
+        for (int u = 0; u < SCAN_ITEMS; ++u) {
+            v[u] = c + u < k ? cnt[(size_t)h * k + c + u] : 0;
+            if (v[u] > SORT_WARP) {
+                const int np = (v[u] + SORT_CTA - 1) / SORT_CTA;
+                const uint64_t range = (uint64_t)((size_t)h * k + c + u) << 32;
+                int at = atomicAdd(lists.len, np);
+                for (int p = 0; p < np; ++p) lists.pieces[at + p] = range | (uint32_t)p;
+                if (np > 1) {
+                    at = atomicAdd(lists.len + 1, np);
+                    for (int p = 0; p < np; ++p) lists.merges[at + p] = range | (uint32_t)p;
+                }
+            }
+        }
         Scan(tmp).ExclusiveSum(v, v, total);
         __syncthreads();
 #pragma unroll
@@ -346,20 +382,18 @@ __global__ void drop_members_kernel(const int32_t* __restrict__ idx, const float
     keys[start[h * k + idx[i]] + a] = ((uint64_t)__float_as_uint(d2[i]) << 32) | (uint32_t)(i - h * n);
 }
 
-// Eight ranges per CTA.  Up to SORT_WARP members: one warp, the rank of a member is the number of smaller keys.
-// Up to SORT_CTA: the CTA sorts the range in shared memory (bitonic).  Longer ones (many equal points): sorted
-// pieces of SORT_CTA, then merged pairwise through the second key array, each member finding its place in the
-// sibling piece by bisection.  Writes the member list and the rank of every point inside its range.
-constexpr int SORT_THREADS = 256, SORT_RANGES = SORT_THREADS / 32, SORT_WARP = 128, SORT_CTA = 4096;
+// The first SORT_PIECE_CTAS (or fewer) CTAs take the pieces of the work list, each sorted in shared memory
+// (bitonic): the whole range, or a run to be merged.  The CTAs behind them take SORT_RANGES ranges each, a warp
+// a range: the rank of a member is the number of smaller keys.  Writes the member list and the rank of every
+// point inside its range.
 __global__ void __launch_bounds__(SORT_THREADS)
 sort_members_kernel(const int32_t* __restrict__ cnt, const int32_t* __restrict__ start, int n, int k, long long n_seg,
-                    uint64_t* __restrict__ keys, uint64_t* __restrict__ keys2, uint32_t* __restrict__ sorted_ids,
+                    int piece_ctas, const MemberLists lists, uint64_t* __restrict__ keys, uint32_t* __restrict__ sorted_ids,
                     int32_t* __restrict__ rank) {
     __shared__ uint64_t sk[SORT_CTA];   // SORT_RANGES x SORT_WARP of it while the warps work
     const int tid = threadIdx.x, warp = tid >> 5, wl = tid & 31;
-    const long long seg0 = (long long)blockIdx.x * SORT_RANGES;
-    {
-        const long long seg = seg0 + warp;
+    if ((int)blockIdx.x >= piece_ctas) {
+        const long long seg = (long long)(blockIdx.x - piece_ctas) * SORT_RANGES + warp;
         const int m = seg < n_seg ? cnt[seg] : 0;
         if (m > 0 && m <= SORT_WARP) {
             const int b = start[seg];
@@ -376,65 +410,104 @@ sort_members_kernel(const int32_t* __restrict__ cnt, const int32_t* __restrict__
                 rank[head + id] = r;
             }
         }
+        return;
     }
-    for (int w = 0; w < SORT_RANGES; ++w) {   // every test below is uniform over the CTA
-        const long long seg = seg0 + w;
-        const int m = seg < n_seg ? cnt[seg] : 0;
-        if (m <= SORT_WARP) continue;
-        const int b = start[seg];
+    const int n_pieces = lists.len[0];
+    for (int e = blockIdx.x; e < n_pieces; e += piece_ctas) {   // every test below is uniform over the CTA
+        const long long seg = (long long)(lists.pieces[e] >> 32);
+        const int p0 = (int)(uint32_t)lists.pieces[e] * SORT_CTA;
+        const int m = cnt[seg], np = min(m - p0, SORT_CTA);
+        const int b = start[seg] + p0;
         const size_t head = (size_t)(seg / k) * n;
-        uint64_t *from = keys + b, *to = keys2 + b;
-        for (int p0 = 0; p0 < m; p0 += SORT_CTA) {
-            const int np = min(m - p0, SORT_CTA);
-            int n2 = 2 * SORT_WARP;
-            while (n2 < np) n2 <<= 1;
-            __syncthreads();
-            for (int i = tid; i < n2; i += SORT_THREADS) sk[i] = i < np ? from[p0 + i] : ~0ull;
-            __syncthreads();
-            for (int size = 2; size <= n2; size <<= 1) {
-                for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                    for (int t = tid; t < n2 / 2; t += SORT_THREADS) {
-                        const int i = 2 * t - (t & (stride - 1)), j = i + stride;
-                        const bool up = (i & size) == 0;
-                        const uint64_t x = sk[i], y = sk[j];
-                        if ((x > y) == up) { sk[i] = y; sk[j] = x; }
-                    }
-                    __syncthreads();
+        int n2 = 2 * SORT_WARP;
+        while (n2 < np) n2 <<= 1;
+        __syncthreads();   // the piece before is written out
+        for (int i = tid; i < n2; i += SORT_THREADS) sk[i] = i < np ? keys[b + i] : ~0ull;
+        __syncthreads();
+        for (int size = 2; size <= n2; size <<= 1) {
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                for (int t = tid; t < n2 / 2; t += SORT_THREADS) {
+                    const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+                    const bool up = (i & size) == 0;
+                    const uint64_t x = sk[i], y = sk[j];
+                    if ((x > y) == up) { sk[i] = y; sk[j] = x; }
                 }
-            }
-            if (m <= SORT_CTA) {
-                for (int i = tid; i < np; i += SORT_THREADS) {
-                    const uint32_t id = (uint32_t)sk[i];
-                    sorted_ids[b + i] = id;
-                    rank[head + id] = i;
-                }
-            } else {
-                for (int i = tid; i < np; i += SORT_THREADS) from[p0 + i] = sk[i];
+                __syncthreads();
             }
         }
-        if (m <= SORT_CTA) continue;
-        for (int len = SORT_CTA; len < m; len *= 2) {
-            __syncthreads();   // the pieces written above (or in the pass before) are visible to the whole CTA
-            const bool last = 2 * (long long)len >= m;
-            for (int i = tid; i < m; i += SORT_THREADS) {
-                const int piece = i / len, sib = piece ^ 1;
-                int lo = min(sib * len, m), hi = min(lo + len, m);
-                const int sib0 = lo;
-                const uint64_t key = from[i];
-                while (lo < hi) {   // members of the sibling piece that come before this one
-                    const int mid = (lo + hi) >> 1;
-                    if (from[mid] < key) lo = mid + 1; else hi = mid;
+        if (m <= SORT_CTA) {
+            for (int i = tid; i < np; i += SORT_THREADS) {
+                const uint32_t id = (uint32_t)sk[i];
+                sorted_ids[b + i] = id;
+                rank[head + id] = i;
+            }
+        } else {
+            for (int i = tid; i < np; i += SORT_THREADS) keys[b + i] = sk[i];
+        }
+    }
+}
+
+// Ranges of more than `len` members, sorted in runs of `len`: up to MERGE_WAYS neighbouring runs become one.  A
+// member's place is its place in its own run and, for each of the others, the number of smaller keys there, found
+// by MERGE_FLIGHT bisections at a time; neighbouring lanes look for neighbouring keys, so most of their reads
+// meet.  The pass that makes a range one run writes the member list and the ranks instead of keys.
+// Bound by the latency of the bisections; what they cost is little beside the build around them: 8 x 131,072 equal
+// bf16 keys, one range a head, 2.31 ms against 2.07 ms of random keys (7.29 ms when the CTA that sorted the pieces
+// of a range also merged them in pairs; 2.75 ms with the radix sort), 8 x 32,768 0.51 and 0.48 ms (1.33; 0.98).
+__global__ void __launch_bounds__(SORT_THREADS)
+merge_members_kernel(const int32_t* __restrict__ cnt, const int32_t* __restrict__ start, int n, int k, int len,
+                     const MemberLists lists, const uint64_t* __restrict__ from_all, uint64_t* __restrict__ to_all,
+                     uint32_t* __restrict__ sorted_ids, int32_t* __restrict__ rank) {
+    grid_wait();
+    const int units = lists.len[1] * (SORT_CTA / MERGE_UNIT);
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        const uint64_t entry = lists.merges[u / (SORT_CTA / MERGE_UNIT)];
+        const long long seg = (long long)(entry >> 32);
+        const int m = cnt[seg];
+        if (m <= len) continue;   // one run already
+        const int i0 = (int)(uint32_t)entry * SORT_CTA + u % (SORT_CTA / MERGE_UNIT) * MERGE_UNIT;
+        const int b = start[seg];
+        const uint64_t* from = from_all + b;
+        const int run = i0 / len, first = run / MERGE_WAYS * MERGE_WAYS;
+        const int runs = min(MERGE_WAYS, (m + len - 1) / len - first);
+        const bool last = (long long)len * MERGE_WAYS >= m;
+        const size_t head = (size_t)(seg / k) * n;
+        for (int i = i0 + threadIdx.x; i < min(i0 + MERGE_UNIT, m); i += SORT_THREADS) {
+            const uint64_t key = from[i];
+            int at = first * len + (i - run * len);
+            for (int s0 = 0; s0 < runs; s0 += MERGE_FLIGHT) {
+                int lo[MERGE_FLIGHT], left[MERGE_FLIGHT];   // what is left to search: left[] keys from lo[] on
+#pragma unroll
+                for (int j = 0; j < MERGE_FLIGHT; ++j) {
+                    const int s = first + s0 + j;
+                    lo[j] = s * len;
+                    left[j] = s0 + j < runs && s != run ? min(len, m - lo[j]) : 0;
+                    at -= left[j] ? lo[j] : 0;
                 }
-                const int at = (piece & ~1) * len + (i - piece * len) + (lo - sib0);
-                if (last) {
-                    const uint32_t id = (uint32_t)key;
-                    sorted_ids[b + at] = id;
-                    rank[head + id] = at;
-                } else {
-                    to[at] = key;
+                for (int reach = len; reach > 0; reach >>= 1) {
+#pragma unroll
+                    for (int j = 0; j < MERGE_FLIGHT; ++j) {
+                        if (left[j] > 0) {
+                            const int half = left[j] >> 1;
+                            const bool below = from[lo[j] + half] < key;
+                            lo[j] += below ? half + 1 : 0;
+                            left[j] = below ? left[j] - half - 1 : half;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < MERGE_FLIGHT; ++j) {
+                    const int s = first + s0 + j;
+                    if (s0 + j < runs && s != run) at += lo[j];
                 }
             }
-            uint64_t* t = from; from = to; to = t;
+            if (last) {
+                const uint32_t id = (uint32_t)key;
+                sorted_ids[b + at] = id;
+                rank[head + id] = at;
+            } else {
+                to_all[b + at] = key;
+            }
         }
     }
 }
@@ -883,7 +956,7 @@ export_kv_kernel(const V* __restrict__ children, int k_pieces, const V* __restri
 // ---------------------------------------------------------------------------
 struct BuildWs {
     size_t total = 0;
-    size_t cents1, cents2, csq, csq_masked, filled, a_idx, a_d2, keys, keys2, rank, sorted, start, count, fill1,
+    size_t cents1, cents2, csq, csq_masked, filled, a_idx, a_d2, keys, keys2, rank, sorted, start, count, pieces, merges, fill1,
         fill2, fbase, lbase, slot1, slot2;
 };
 
@@ -907,7 +980,9 @@ static BuildWs carve(const hira_index_t* ix, int n_keys) {
     w.rank = take(H * n * 4);
     w.sorted = take(H * n * 4);
     w.start = take(H * k1 * 4);
-    w.count = take(H * k1 * 4);
+    w.count = take((H * k1 + MEMBER_LISTS) * 4);
+    w.pieces = take(pieces_bound(H * n) * 8);
+    w.merges = take(merges_bound(H * n) * 8);
     w.fill1 = take(H * k1 * 4);
     w.fill2 = take(H * k2 * 4);
     w.fbase = take(H * (k1 + 1) * 4);
@@ -944,15 +1019,25 @@ static int build_level(int dtype, const T* points, long long p_head_stride, int 
         HIRA_CHECK_LAUNCH("gather centres launch");
     }
     const int blocks = (int)((total + 255) / 256);
+    const MemberLists lists{reinterpret_cast<uint64_t*>(base + w.pieces), reinterpret_cast<uint64_t*>(base + w.merges), count + n_seg};
+    const size_t most = pieces_bound((size_t)total);
+    const int piece_ctas = most < (size_t)SORT_PIECE_CTAS ? (int)most : SORT_PIECE_CTAS;
     // counts, ranges and ranks of the points' latest assignment; `placed`: the slots of the points to leave out
     auto sort_members = [&](const int32_t* placed) -> int {
-        if (placed) cudaMemsetAsync(count, 0, (size_t)n_seg * 4, s);   // else cleared with the norms of the centres
+        if (placed) cudaMemsetAsync(count, 0, ((size_t)n_seg + MEMBER_LISTS) * 4, s);   // else cleared with the norms of the centres
         count_members_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, placed, count, rank, status);
-        member_starts_kernel<<<n_heads, 1024, 0, s>>>(count, n, k, start);
+        member_starts_kernel<<<n_heads, 1024, 0, s>>>(count, n, k, start, lists);
         drop_members_kernel<<<blocks, 256, 0, s>>>(a_idx, a_d2, n, k, total, start, rank, keys);
-        const long long sblocks = (n_seg + SORT_RANGES - 1) / SORT_RANGES;
-        sort_members_kernel<<<(unsigned)sblocks, SORT_THREADS, 0, s>>>(count, start, n, k, n_seg, keys, keys2, sorted, rank);
+        const long long sblocks = piece_ctas + (n_seg + SORT_RANGES - 1) / SORT_RANGES;
+        sort_members_kernel<<<(unsigned)sblocks, SORT_THREADS, 0, s>>>(count, start, n, k, n_seg, piece_ctas, lists, keys, sorted, rank);
         HIRA_CHECK_LAUNCH("member sort launch");
+        uint64_t *from = keys, *to = keys2;
+        for (long long len = SORT_CTA; len < n; len *= MERGE_WAYS) {   // what a range of all the points would take
+            const cudaError_t e = launch_chained(merge_members_kernel, dim3(4 * SM_COUNT), dim3(SORT_THREADS), 0, s, (const int32_t*)count,
+                                                 (const int32_t*)start, n, k, (int)len, lists, (const uint64_t*)from, to, sorted, rank);
+            if (e != cudaSuccess) { set_error("member merge launch: %s", cudaGetErrorString(e)); return HIRA_ERR_CUDA; }
+            uint64_t* t = from; from = to; to = t;
+        }
         return HIRA_OK;
     };
     const int iters = n_iters < 1 ? 1 : n_iters;

@@ -49,6 +49,9 @@ void set_error(const char* fmt, ...);
 
 int validate_index(const hira_index_t* ix, bool need_values);
 
+constexpr int SM_COUNT = 148;   // of a B200
+
+
 // Programmatic launches.  The kernels of one decode step follow each other on one stream; launched with
 // launch_chained, a kernel's CTAs may become resident while the kernel before it still runs, so that the
 // launch latency and the prologue are not on the step's critical path.  A kernel launched so calls

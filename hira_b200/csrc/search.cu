@@ -739,7 +739,7 @@ extern "C" int hira_search_tile_parents(const hira_index_t* ix) {
     const bool q8 = ix->children_q8 && ix->dim == 128 && bf >= 8 && (tp * bf) % 128 == 0 && ix->cap_parents % tp == 0;
     if (!q8 && ix->n_heads >= 1) {
         auto ctas = [&](int t) { return (long long)ix->n_heads * ((ix->cap_parents + t - 1) / t); };
-        while (ctas(tp) < 2 * 148 && tp * bf > 256) {
+        while (ctas(tp) < 2 * SM_COUNT && tp * bf > 256) {
             int next;
             if (ix->depth == 2) next = (tp + 1) / 2;
             else if (tp > bf) next = (tp / bf + 1) / 2 * bf;   // whole grandparents
