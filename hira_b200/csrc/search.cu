@@ -734,12 +734,21 @@ extern "C" int hira_search_tile_parents(const hira_index_t* ix) {
     // one CTA from its gates to its last row, so with few of them the length of that walk is the time of the
     // search.  Two CTAs per SM are aimed for, 256 rows are where the fixed part of a CTA takes over.
     // Measured, whole decode step: 12 heads of 9,001 keys (D = 64, bf = 16) 41.4 us with 1024 rows (108 CTAs),
-    // 39.6 with 512, 35.4 with 256 (432 CTAs), 38.0 with 128.  The int8 pre-filter gains nothing from it
-    // (8 heads of 2,048 keys 27.5, 26.3, 27.4, 30.2 us; 32,768 keys 40.3, 42.3, 46.7, 57.0 us) and keeps its tiles.
+    // 39.6 with 512, 35.4 with 256 (432 CTAs), 38.0 with 128.  Rows of 512 bytes and more keep the memory busy from
+    // fewer CTAs.  Dense search out of DRAM, 8 key heads, tiles of 1024 and of 512 rows: 224 CTAs of 1024 rows (4 query
+    // heads each, 200 fp32 channels) 127.0 and 106.9 us, 248 (1; 256 bf16 channels) 39.7 and 37.4, but 256 (4; 200
+    // fp32) 128.5 and 132.7, 256 (4; 256 bf16) 57.6 and 62.9, 288 (1; 200 fp32) 88.4 and 103.4; of 512 and of 256
+    // rows, 256 CTAs of 512 rows (4; 200 fp32) 71.5 and 77.7, (4; 256 bf16) 36.4 and 42.4.  Below 512 bytes 256 CTAs
+    // of 1024 rows are still too few: 64 bf16 channels 25.6 and 21.7 us, 64 fp32 38.0 and 39.0, out of L2 26.2 and
+    // 23.6.  The number of query heads is not known here; where D > 128 a third one brings a second CTA per tile, and
+    // larger tiles would do (128 CTAs, 4; 256 bf16: 33.6 and 36.4 us, but with 1: 31.7 and 25.2).
+    // The int8 pre-filter gains nothing from it (8 heads of 2,048 keys 27.5, 26.3, 27.4, 30.2 us; 32,768 keys 40.3,
+    // 42.3, 46.7, 57.0 us) and keeps its tiles.
     const bool q8 = ix->children_q8 && ix->dim == 128 && bf >= 8 && (tp * bf) % 128 == 0 && ix->cap_parents % tp == 0;
     if (!q8 && ix->n_heads >= 1) {
         auto ctas = [&](int t) { return (long long)ix->n_heads * ((ix->cap_parents + t - 1) / t); };
-        while (ctas(tp) < 2 * SM_COUNT && tp * bf > 256) {
+        const long long enough = (long long)ix->dim * elem_size(ix->dtype) >= 512 ? 250 : 2 * SM_COUNT;
+        while (ctas(tp) < enough && tp * bf > 256) {
             int next;
             if (ix->depth == 2) next = (tp + 1) / 2;
             else if (tp > bf) next = (tp / bf + 1) / 2 * bf;   // whole grandparents

@@ -244,3 +244,12 @@ def test_threshold_samples_are_at_least_one_and_at_most_the_keys(sample_size, wa
         rows = _samples_for(ix, sample_size)
         assert rows.shape == (4, want, 64) and bool((rows == 1.0).all())
         assert _samples_for(ix, sample_size).shape == rows.shape
+
+
+@pytest.mark.parametrize("dim,dtype,cap,rows", [(64, torch.float32, 1024, 512), (64, torch.bfloat16, 1024, 512), (64, torch.float32, 512, 256),
+                                                (200, torch.float32, 1024, 1024), (200, torch.float32, 896, 512), (200, torch.float32, 512, 512),
+                                                (128, torch.float32, 1024, 1024), (256, torch.bfloat16, 992, 512), (256, torch.bfloat16, 480, 256),
+                                                (64, torch.float32, 32, 256), (256, torch.bfloat16, 32, 256)])
+def test_tile_size_follows_the_bytes_of_a_row(dim, dtype, cap, rows):
+    """8 heads of branching 32: tiles are halved while they are too few to keep the memory busy, of long rows fewer."""
+    assert S.tile_parents(_state(dim, cap_parents=cap, dtype=dtype)) * 32 == rows
