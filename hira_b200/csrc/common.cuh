@@ -418,7 +418,7 @@ __device__ __forceinline__ void load_vec(const T* v, float (&b)[NCH][8], int lan
 // ---------------------------------------------------------------------------
 // Both quotients are defined as correctly rounded divisions, but a division per element and quotient was
 // most of the quantisation's time.  So they are formed with reciprocals (of the scales once for all rows of
-// a group, of the step once a row), which is within 4e-7 of the quotient, and divided out only where that
+// a group, of the step once a row), within 3.6e-7 (6 x 2^-24) of the quotient, and divided out only where that
 // could round differently: a step whose fp16 neighbours are in question, a quotient next to half an integer.
 // The stored step and integers are those of the divisions; err takes the residual of the k' at hand, whose
 // own rounding (2^-22 of ||q|| ||x|| at most) lies far inside its second term.
@@ -500,7 +500,9 @@ __device__ __forceinline__ void q8_write_row(const float (&x)[2][8], const float
             off = fmaxf(off, fabsf(__fsub_rn(t, __fsub_rn(kr[i][e], Q8_ROUND))));
         }
     }
-    if (off > 0.49995f && ok) {   // the quotients are off by 127 x 4e-7 at most: divide what lies that close to a tie
+    // Two reciprocals and two products here, two divisions there: 6 roundings of 2^-24, 127 x 6 x 2^-24 = 4.6e-5 at most
+    // between the quotients.  What lies closer to a tie than 5e-5 is divided.
+    if (off > 0.49995f && ok) {
         q8_quotients(x, chan, lane, step, kr);
 #pragma unroll
         for (int i = 0; i < 2; ++i)

@@ -274,3 +274,55 @@ def test_build_time_does_not_depend_on_how_crowded_a_centre_is():
             best = min(best, a.elapsed_time(b))
         ms.append(best)
     assert ms[1] < 2 * ms[0], ms      # measured 1.1; 3.6 when one block sorted and merged a whole range
+
+
+def test_int8_copy_next_to_ties_is_that_of_divisions():
+    """Rows whose largest channel lies within a few roundings of 127 fp16 steps and whose others lie as close to half a
+    step: the stored step and integers are those of k' = k / s, step = max |k'| / 127 rounded up to fp16,
+    rint(k' / step) by divisions, both from the whole copy being made and from appends."""
+    h, bf, d, cap = 2, 32, 128, 544
+    n = cap * bf                                   # more than 16,384 slots: every other one is sampled for the scales
+    keys = make_keys(h, n, d, 71, normalize=False)
+    st = S.IndexState(n_heads=h, dim=d, vdim=d, bf=bf, depth=2, cap_parents=cap + 300, dtype=torch.float32, vdtype=torch.float32, device="cuda",
+                      with_values=False)
+    S.build(st, keys, None)
+    scale = st.q8_chan_scale[:, None, :d].double()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda lo, hi, *s: torch.randint(lo, hi + 1, s, generator=g, device="cuda").double()   # noqa: E731
+
+    def rows(m):
+        step = (rnd(1024, 2047, h, m, 1) * 2.0 ** rnd(-22, -14, h, m, 1))                        # an fp16 number
+        k = (rnd(-127, 126, h, m, d) + 0.5) * step * (1 + rnd(-12, 12, h, m, d) * 2.0 ** -24)
+        top = rnd(0, d - 1, h, m, 1).long()
+        k.scatter_(2, top, 127 * step * (1 + rnd(-4, 4, h, m, 1) * 2.0 ** -24))
+        return (k * scale).float()
+
+    def check(j, slots):
+        c = st.q8_chan_scale[j, :d]
+        kp = st.children[j, slots] / c
+        amax = kp.abs().amax(dim=-1)
+        step = amax / torch.full_like(amax, 127.0)      # a tensor: by a number, torch multiplies with its reciprocal
+        h16 = step.half()
+        h16 = torch.where(h16.float() < step, torch.nextafter(h16, torch.full_like(h16, float("inf"))), h16)
+        meta = st.children_q8_meta[j, slots]
+        assert torch.equal((meta & 0xffff).to(torch.int16).view(torch.float16), h16)
+        quot = kp / h16.float()[:, None]
+        want = torch.round(quot).clamp(-127, 127)
+        place = torch.arange(8, device="cuda")[None, :] ^ (slots & 7)[:, None]                   # 16-byte chunk i of slot r at i ^ (r & 7)
+        got = st.children_q8[j, slots].view(-1, 8, 16).gather(1, place[:, :, None].expand(-1, -1, 16)).reshape(want.shape)
+        assert torch.equal(got, want.to(torch.int8))
+        err = (meta >> 16 & 0xffff).to(torch.int16).view(torch.float16).double()
+        assert bool((err >= (st.children[j, slots].double() / c.double() - want.double() * h16.double()[:, None]).norm(dim=-1)).all())
+        return int(((quot.frac().abs() - 0.5).abs() < 5e-5).sum())
+
+    odd = torch.arange(1, n, 2, device="cuda")
+    st.children[:, odd] = rows(len(odd))
+    L.check(L.load().hira_q8_refresh(st.struct, L.current_stream()))
+    assert min(check(j, odd) for j in range(h)) > 100_000
+    new = rows(256)
+    for i in range(0, 256, 32):
+        S.append(st, new[:, i:i + 32].contiguous(), None)
+    assert int(st.status) == 0
+    for j in range(h):
+        slots = (st.slot2token[j] >= n).nonzero()[:, 0]
+        assert len(slots) == 256 and check(j, slots) > 4000
