@@ -451,16 +451,24 @@ static int launch_append(const AppendParams& P, cudaStream_t s) {
 
 using namespace hira;
 
+// Slices of a head's parents in the staged path; with three levels one more CTA takes the grandparents.  Two CTAs fit
+// an SM, and what counts is that all of them are resident at once: as many slices as that allows, two at least.
+// us an append, bf16 rows of 128 channels, branching 32, three levels (before: up to nine slices a head where fewer
+// would have been resident): 32 heads of 32,768 keys 13.7 -> 12.4, 64 18.9 -> 14.4, 128 28.7 -> 19.2, 256 42.0 -> 34.5.
+// Slices of more than 1,536 rows outlast a second wave of at least five: 80 heads of 131,072 keys 34.6 -> 29.7
+// (but 128 heads, three slices against two: 48.4 and 42.9).  Up to 512 parents one slice will do where two do not
+// fit: 128 heads of 2,048 keys 14.8 -> 12.9, 400 30.3 -> 26.0.
 static int append_parts(const hira_index_t* ix) {
-    // two CTAs per SM, all resident at once, where that leaves enough slices; with many heads several waves of
-    // shorter ones; slices of at least 128 parents
-    int parts = 2 * SM_COUNT / ix->n_heads - 1;
-    if (parts < 9) parts = (8 * SM_COUNT + ix->n_heads - 1) / ix->n_heads < 9 ? (8 * SM_COUNT + ix->n_heads - 1) / ix->n_heads : 9;
+    auto waves = [&](int w) { return w * 2 * SM_COUNT / ix->n_heads - (ix->depth == 3 ? 1 : 0); };
+    const int least = ix->depth == 3 && ix->cap_parents <= 512 ? 1 : 2;
+    int parts = waves(1) > least ? waves(1) : least;
+    if (ix->cap_parents / parts > 1536 && waves(2) >= 5) parts = waves(2);
     const int max_parts = ix->cap_parents / 128;
     if (parts > max_parts) parts = max_parts;
     if (parts > 64) parts = 64;
     return parts < 1 ? 1 : parts;
 }
+static bool staged_pays(const hira_index_t* ix) { return ix->cap_parents >= 256; }   // two slices' worth of parents
 
 extern "C" size_t hira_append_workspace_bytes(const hira_index_t* ix, int32_t n_new) {
     if (!ix || n_new < 1 || n_new > APPEND_MAX_STAGED || ix->n_heads < 1 || ix->cap_parents < 1) return 0;
@@ -499,7 +507,7 @@ extern "C" int hira_append(const hira_index_t* ix, const void* new_k, const void
     P.bf_magic = (ix->bf > 1 && ix->cap_parents < (1 << 20))
                      ? (uint32_t)((0x100000000ull + (uint64_t)ix->bf - 1) / (uint64_t)ix->bf) : 0u;
     const size_t need = hira_append_workspace_bytes(ix, n_new);
-    if (workspace != nullptr && need > 0 && workspace_bytes >= need && append_parts(ix) > 1) {
+    if (workspace != nullptr && need > 0 && workspace_bytes >= need && staged_pays(ix)) {
         P.partial = reinterpret_cast<BestRec*>(workspace);
         P.n_parts = append_parts(ix);
     }

@@ -292,8 +292,8 @@ int hira_exchange_merge(const float* local_rows, void* const* peer_bufs,
  *   status: device int32, OR-ed with HIRA_STATUS_* on capacity exhaustion
  *   workspace: optional scratch of hira_append_workspace_bytes(index, n_new)
  *          bytes (0 = not applicable, for n_new > 32).  With it the parent scan is
- *          spread over the whole GPU (one kernel scans slices, a second one picks
- *          the arg-min and inserts); without it (NULL) one CTA per head does
+ *          spread over the whole GPU (many CTAs scan slices, the last one of a head
+ *          picks the arg-min and inserts); without it (NULL) one CTA per head does
  *          everything.  The result is identical either way.
  */
 size_t hira_append_workspace_bytes(const hira_index_t* index, int32_t n_new);

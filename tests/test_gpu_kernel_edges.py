@@ -326,3 +326,15 @@ def test_int8_copy_next_to_ties_is_that_of_divisions():
     for j in range(h):
         slots = (st.slot2token[j] >= n).nonzero()[:, 0]
         assert len(slots) == 256 and check(j, slots) > 4000
+
+
+@pytest.mark.parametrize("h,depth,bf,n,m", [(300, 3, 8, 2000, 1), (150, 3, 8, 2000, 3), (100, 3, 4, 3000, 1), (200, 2, 4, 2500, 2), (3, 3, 4, 1000, 1), (3, 2, 4, 1000, 4)])
+def test_staged_append_of_many_heads_matches_oracle(h, depth, bf, n, m):
+    """One slice a head beside the grandparents', two, several, and indexes too small for slices."""
+    d = 8
+    st, ox, _, _ = build_both(h, n, d, bf, depth, torch.float32, seed=41, spare=bf * 4)
+    for r in range(2):
+        nk, nv = make_keys(h, m, d, 60 + r), make_keys(h, m, d, 70 + r, normalize=False)
+        S.append(st, nk, nv)
+        O.append(ox, nk, nv)
+    assert_index_equal(st, ox, "many heads")

@@ -253,3 +253,14 @@ def test_threshold_samples_are_at_least_one_and_at_most_the_keys(sample_size, wa
 def test_tile_size_follows_the_bytes_of_a_row(dim, dtype, cap, rows):
     """8 heads of branching 32: tiles are halved while they are too few to keep the memory busy, of long rows fewer."""
     assert S.tile_parents(_state(dim, cap_parents=cap, dtype=dtype)) * 32 == rows
+
+
+@pytest.mark.parametrize("heads,cap,depth,parts", [(1, 4096, 3, 32), (1, 32768, 2, 64), (8, 4096, 3, 32), (8, 32768, 3, 36), (32, 1024, 3, 8), (32, 1024, 2, 8),
+                                                   (32, 2048, 2, 9), (64, 1024, 3, 3), (128, 1024, 3, 2), (128, 512, 3, 1), (128, 4096, 3, 2), (128, 512, 2, 2),
+                                                   (80, 4096, 3, 6), (80, 1024, 3, 2), (400, 512, 3, 1), (400, 4096, 3, 2), (8, 128, 3, 1)])
+def test_append_slices_fit_the_gpu_at_once(heads, cap, depth, parts):
+    """The workspace holds one result of 8 bytes a slice and one of the grandparents, per key and head."""
+    st = _state(8, n_heads=heads, bf=8, depth=depth, cap_parents=cap)
+    for m in (1, 32):
+        assert L.load().hira_append_workspace_bytes(st.struct, m) == heads * m * (parts + 1) * 8
+    assert L.load().hira_append_workspace_bytes(st.struct, 33) == 0
