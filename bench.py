@@ -620,7 +620,7 @@ def secondary_cfg3(args, dev):
             "append_us_per_step": statistics.mean(append_us), "append_us_by_window": append_us,
             "append_algorithmic_bytes": append_bytes, "rebuild_ms": statistics.median(rebuild_ms) if rebuild_ms else None, "rebuild_ms_each": rebuild_ms,
             "rebuilds": len(rebuild_ms), "initial_build_ms": build_ms,
-            "note": "append step = 8 heads, launch-latency bound (one small kernel pair per step)"}
+            "note": "append step = 8 heads, launch-latency bound (one small kernel per step)"}
 
 
 def secondary_cfg4(args, dev, rank, world, dist, barrier, peak):

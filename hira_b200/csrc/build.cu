@@ -29,16 +29,8 @@ int launch_assign_tc(const void* points, long long p_head_stride, const void* ce
 bool assign_tc_supported(int dtype, int n, int k, int dim);
 
 // ---------------------------------------------------------------------------
-// Sequential-chain helpers (the assignment's arithmetic: one fp32 FMA chain
-// over d = 0..D-1 starting from 0).
+// The assignment's arithmetic: one fp32 FMA chain over d = 0..D-1 starting from 0.
 // ---------------------------------------------------------------------------
-template <typename T> __device__ __forceinline__ float to_f(T v);
-template <> __device__ __forceinline__ float to_f(float v) { return v; }
-template <> __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename T> __device__ __forceinline__ T from_f(float v);
-template <> __device__ __forceinline__ float from_f(float v) { return v; }
-template <> __device__ __forceinline__ __nv_bfloat16 from_f(float v) { return __float2bfloat16_rn(v); }
-
 template <typename T>
 __device__ __forceinline__ void memcpy_chunk(RawChunk<T>& raw, const T* src) {
     T e[8];
