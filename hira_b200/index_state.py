@@ -75,8 +75,10 @@ class IndexState:
         else:
             self.children_q8 = self.children_q8_meta = self.q8_chan_scale = self.q8_query_scratch = None
         self.status = z((1,), dtype=torch.int32, device=dev)
+        self.arrays_device = self.status.device     # with its index, which `device` may lack
         self._struct = None
         self._append_bytes = {}
+        self._append_ws = None, 0      # scratch of the appends, and the stream it was allocated on
         # streams the arrays are kept alive for: the one they are allocated on, and those of `used_on`
         self._streams = {L.current_stream(dev)} if dev.type == "cuda" else set()
         self._active_parents = 0
@@ -203,6 +205,14 @@ class CompactResult:
     tile_rows: int
     n_tiles_active: Optional[int] = None   # tiles the last search wrote (None: all)
 
+    def __post_init__(self):
+        """What a search has to be like for these buffers to take its output (compact_fits), None if nothing can."""
+        hq, slots = self.idx.shape
+        bf = self.tile_rows // self.tile_parents
+        whole = (self.score.shape == self.idx.shape and bf * self.tile_parents == self.tile_rows
+                 and self.count.shape == (hq, -(-(slots // bf) // self.tile_parents)))
+        self.made_for = (hq, slots, bf, self.tile_parents, self.idx.device) if whole else None
+
     def to_lists(self):
         """Per query head: (slots, scores) as 1-D CPU tensors, ascending slot order."""
         idx, score, count = self.idx.cpu(), self.score.cpu(), self.count.cpu()
@@ -304,8 +314,7 @@ def alloc_compact(st: IndexState, hq: int, tp: Optional[int] = None) -> CompactR
 def compact_fits(st: IndexState, hq: int, c: CompactResult, tp: int) -> bool:
     """Whether `c` can take what a search of `st` by `hq` heads in tiles of `tp` parents writes.  The tile size
     is part of that: two indexes of equal capacity need not have the same."""
-    return (c.tile_parents == tp and c.tile_rows == tp * st.bf and c.idx.device == st.children.device
-            and c.idx.shape == c.score.shape == (hq, st.cap_children) and c.count.shape == (hq, n_tiles(st, tp)))
+    return c.made_for == (hq, st.cap_children, st.bf, tp, st.arrays_device)
 
 
 def _check_compact(st: IndexState, hq: int, c: CompactResult, tp: int):
@@ -334,15 +343,18 @@ def queue_stride(t: torch.Tensor) -> Optional[int]:
     """Elements between the heads of a (B, H, n, D) or (H, n, D) queue whose rows lie one behind another from
     a 16-byte boundary -- a whole tensor or the filled part of a queue buffer --, None for any other layout.
     A stride along a dimension of one says nothing and is not looked at."""
-    (h, n, d), (hs, ns, ds) = t.shape[-3:], t.stride()[-3:]
-    b, bs = (t.shape[0], t.stride(0)) if t.ndim == 4 else (1, 0)
-    if h == 1:                       # the heads to step over are the batch
-        h, hs, b = b, bs, 1
+    shape, strides = t.shape, t.stride()
+    h, n, d, hs = shape[-3], shape[-2], shape[-1], strides[-3]
+    if t.ndim == 4 and shape[0] > 1:
+        if h == 1:                   # the heads to step over are the batch
+            h, hs = shape[0], strides[0]
+        elif strides[0] != h * hs:
+            return None
     if h == 1:
         hs = n * d
-    if ds != 1 or (n > 1 and ns != d) or hs < n * d or t.data_ptr() % 16 or hs * t.element_size() % 16:
+    if strides[-1] != 1 or (n > 1 and strides[-2] != d) or hs < n * d or t.data_ptr() % 16 or hs * t.element_size() % 16:
         return None
-    return hs if b == 1 or bs == h * hs else None
+    return hs
 
 
 def dense_rows(t: torch.Tensor, dtype: torch.dtype, device) -> torch.Tensor:
@@ -415,21 +427,20 @@ def append(st: IndexState, new_k: torch.Tensor, new_v: Optional[torch.Tensor], t
     _check_rows(new_k, st.n_heads, m, st.dim, st.dtype)
     if new_v is not None:
         _check_rows(new_v, st.n_heads, m, st.vdim, st.vdtype)
-    ws, nbytes = None, 0
+    ws, nbytes, stream = None, 0, L.current_stream(st.device)
     if use_workspace:
         sizes = st._append_bytes     # depends on the heads, the capacity and m only
         nbytes = sizes.get(m)
         if nbytes is None:
             nbytes = sizes[m] = int(lib.hira_append_workspace_bytes(st.struct, m))
         if nbytes:
-            ws, home = getattr(st, "_append_ws", (None, 0))
-            stream = L.current_stream(st.device)
+            ws, home = st._append_ws
             if ws is None or ws.numel() < nbytes or home != stream:    # scratch of the stream it is used on
                 ws = torch.empty((nbytes,), dtype=torch.uint8, device=st.device)
                 st._append_ws = ws, stream
     rc = lib.hira_append(st.struct, L.ptr(new_k), L.ptr(new_v), m, m * st.dim,
                          m * st.vdim if new_v is not None else 0, token_base, L.ptr(st.status),
-                         L.ptr(ws), nbytes, L.current_stream(st.device))
+                         L.ptr(ws), nbytes, stream)
     L.check(rc, "hira_append")
 
 
