@@ -1025,11 +1025,12 @@ __global__ void q8_chan_finish_kernel(const hira_index_t ix) {
 // one 8-lane group quantises Q8_QUANT_ROWS slots (see q8_write_row in common.cuh), two bf16 rows in flight.
 // Bound by the instructions of a row (about 500 a warp of four rows), not by its D e + 132 bytes: three CTAs
 // per SM in 80 registers issue more of them than two with four rows in flight each (61 us at half the issue
-// rate).  8 x 32,768 bf16 rows: 59.3 -> 50.7 us (one row per group with its 32 divisions before).
-constexpr int Q8_QUANT_ROWS = 8, Q8_QUANT_THREADS = 256;
+// rate).  8 x 32,768 bf16 rows: 59.3 -> 50.7 us (one row per group with its 32 divisions before).  An index too small to
+// give every SM a CTA of that is shared out by fewer rows a group (Q8_QUANT_SMALL).
+constexpr int Q8_QUANT_ROWS = 8, Q8_QUANT_LEAST = 2, Q8_QUANT_THREADS = 256;
 template <typename T>
 __global__ void __launch_bounds__(Q8_QUANT_THREADS, 3)
-q8_quantize_kernel(const hira_index_t ix, const size_t slots_bound) {
+q8_quantize_kernel(const hira_index_t ix, const size_t slots_bound, const int rows) {
     constexpr int FLIGHT = 4 / (int)sizeof(T);
     const int lane = threadIdx.x & (GROUP - 1);
     const size_t capC = (size_t)ix.cap_parents * ix.bf;
@@ -1038,13 +1039,13 @@ q8_quantize_kernel(const hira_index_t ix, const size_t slots_bound) {
     size_t n_slots = (size_t)(ix.depth == 3 ? ix.used[h * 4 + 1] * ix.bf : ix.used[h * 4 + 0]) * ix.bf;
     n_slots = n_slots < slots_bound ? n_slots : slots_bound;
     constexpr int GROUPS = Q8_QUANT_THREADS / GROUP;
-    const size_t slot0 = (size_t)blockIdx.x * (GROUPS * Q8_QUANT_ROWS) + threadIdx.x / GROUP;   // then every GROUPS-th
+    const size_t slot0 = (size_t)blockIdx.x * (GROUPS * rows) + threadIdx.x / GROUP;   // then every GROUPS-th
     if (slot0 >= n_slots) return;
     const float* chan = ix.q8_chan_scale + (size_t)h * HIRA_Q8_CHAN;
     float inv[2][8];
     q8_load_inv_scales(chan, inv, lane);
     const float slack = q8_slack(chan);
-    for (int r0 = 0; r0 < Q8_QUANT_ROWS; r0 += FLIGHT) {
+    for (int r0 = 0; r0 < rows; r0 += FLIGHT) {   // rows: Q8_QUANT_LEAST or a multiple of it
         RawChunk<T> raw[FLIGHT][2];
 #pragma unroll
         for (int u = 0; u < FLIGHT; ++u) {
@@ -1076,18 +1077,20 @@ int q8_refresh(const hira_index_t* ix, cudaStream_t s, long long parents_bound) 
                    "the int8 side copy needs dim == 128 and its meta / channel-scale arrays");
     if (parents_bound <= 0 || parents_bound > ix->cap_parents) parents_bound = ix->cap_parents;
     const size_t slots_bound = (size_t)parents_bound * ix->bf;
-    constexpr size_t per_block = Q8_QUANT_THREADS / GROUP * Q8_QUANT_ROWS;
-    const dim3 blocks((unsigned)((slots_bound + per_block - 1) / per_block), (unsigned)ix->n_heads);
+    auto blocks_of = [&](int rows) { return (slots_bound + Q8_QUANT_THREADS / GROUP * rows - 1) / (Q8_QUANT_THREADS / GROUP * rows); };
+    int rows = Q8_QUANT_ROWS;
+    while (rows > Q8_QUANT_LEAST && blocks_of(rows) * ix->n_heads < (size_t)SM_COUNT) rows /= 2;
+    const dim3 blocks((unsigned)blocks_of(rows), (unsigned)ix->n_heads);
     cudaMemsetAsync(ix->q8_chan_scale, 0, (size_t)ix->n_heads * HIRA_Q8_CHAN * sizeof(float), s);
     const dim3 parts(Q8_CHAN_PARTS, (unsigned)ix->n_heads);
     if (ix->dtype == HIRA_BF16) {
         q8_chan_sums_kernel<__nv_bfloat16><<<parts, Q8_DIM, 0, s>>>(*ix);
         q8_chan_finish_kernel<<<ix->n_heads, Q8_DIM, 0, s>>>(*ix);
-        q8_quantize_kernel<__nv_bfloat16><<<blocks, Q8_QUANT_THREADS, 0, s>>>(*ix, slots_bound);
+        q8_quantize_kernel<__nv_bfloat16><<<blocks, Q8_QUANT_THREADS, 0, s>>>(*ix, slots_bound, rows);
     } else {
         q8_chan_sums_kernel<float><<<parts, Q8_DIM, 0, s>>>(*ix);
         q8_chan_finish_kernel<<<ix->n_heads, Q8_DIM, 0, s>>>(*ix);
-        q8_quantize_kernel<float><<<blocks, Q8_QUANT_THREADS, 0, s>>>(*ix, slots_bound);
+        q8_quantize_kernel<float><<<blocks, Q8_QUANT_THREADS, 0, s>>>(*ix, slots_bound, rows);
     }
     HIRA_CHECK_LAUNCH("int8 side copy launch");
     return HIRA_OK;
