@@ -9,6 +9,7 @@
 // largest score over a whole head (used to set tau so that a given number of
 // keys survives).
 #include "common.cuh"
+#include <type_traits>
 #include <math_constants.h>
 
 namespace hira {
@@ -49,13 +50,14 @@ __device__ __forceinline__ uint32_t warp_merge_top(uint32_t a, uint32_t b, int w
 // Scores travel as order-preserving integers; a NaN score sorts last.
 // Measured, 1000 bf16 samples, D = 128, k = 16: 32.3 -> 8.4 us for 32 query heads (256 threads, one row in
 // flight per group and a 55-step bitonic sort before), 42.0 -> 8.9 us for 64.
-template <typename T, int NCH, int TH>
-__global__ void __launch_bounds__(TH)
+template <typename T, int NCH, int TH, int PER_SM>
+__global__ void __launch_bounds__(TH, PER_SM)
 threshold_kernel(const T* __restrict__ samples, long long head_stride, int n_samples, int dim,
                  const float* __restrict__ q, const int32_t* __restrict__ q2kv, int group, int method, int k,
                  float* __restrict__ tau_out) {
     constexpr int HW = TH / GROUP;
-    constexpr int ROWS = 16 / ((int)sizeof(T) * NCH);   // 128 bytes of rows in flight per lane
+    // 128 bytes of rows in flight per lane; 64 of wide bf16 rows where four CTAs are to fit an SM
+    constexpr int ROWS = NCH == 4 && PER_SM == 4 ? 1 : 16 / ((int)sizeof(T) * NCH);
     __shared__ uint32_t s[TAU_MAX_SAMPLES];
     const int tid = threadIdx.x, lane = tid & (GROUP - 1), hw = tid / GROUP, warp = tid >> 5, wl = tid & 31;
     grid_wait();
@@ -254,15 +256,30 @@ extern "C" int hira_threshold(const void* samples, int32_t dtype, int32_t n_head
     const bool wide = dim > 128;  // chunks per lane: 2 up to 128 elements, else 4
     const dim3 grid((unsigned)n_qheads);
     cudaError_t e;
-    if (dtype == HIRA_BF16) {
-        auto* p = reinterpret_cast<const __nv_bfloat16*>(samples);
-        if (wide) e = launch_chained(threshold_kernel<__nv_bfloat16, 4, 512>, grid, dim3(512), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
-        else e = launch_chained(threshold_kernel<__nv_bfloat16, 2, 1024>, grid, dim3(1024), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
-    } else {
-        auto* p = reinterpret_cast<const float*>(samples);
-        if (wide) e = launch_chained(threshold_kernel<float, 4, 512>, grid, dim3(512), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
-        else e = launch_chained(threshold_kernel<float, 2, 1024>, grid, dim3(1024), 0, s, p, (long long)head_stride, n_samples, dim, q, q2kv, group, method, k, tau_out);
-    }
+    auto run = [&](auto kern, const auto* rows, int threads) {
+        e = launch_chained(kern, grid, dim3((unsigned)threads), 0, s, rows, (long long)head_stride, (int)n_samples, (int)dim, q, q2kv,
+                           group, (int)method, (int)k, tau_out);
+    };
+    // One CTA a query head, and as many threads as leave all CTAs resident: 1024 while there is an SM for each,
+    // smaller ones beyond that and for few samples.  bf16 samples of 128 channels, us with 1024, 512 and 256 threads:
+    // 128 heads x 1,000, k = 16: 8.3, 9.1, 12.4;  256 heads 15.5, 12.6, 13.9;  512 heads 29.7, 23.4, 21.4 (k = 33,
+    // 62.6, 51.0, 47.1);  512 heads x 16: 14.6, 7.3, 4.1;  32 heads x 100: 4.7, 3.8, 3.5;  384 heads x 4,096 64, 67,
+    // 76 (k = 82, 174, 179, 212).  Rows above 128 channels (200): 512 heads x 1,000, k = 33 85 with 512 threads, 73
+    // with 256 of three CTAs an SM, 57 with four;  384 heads 64, 45, 56.
+    auto sized = [&](const auto* rows) {
+        typedef typename std::remove_const<typename std::remove_pointer<decltype(rows)>::type>::type T;
+        if (wide) {
+            if (n_qheads > 3 * SM_COUNT) run(threshold_kernel<T, 4, 256, 4>, rows, 256);
+            else if (n_qheads > (n_samples <= 128 ? 1 : 2) * SM_COUNT) run(threshold_kernel<T, 4, 256, 3>, rows, 256);
+            else run(threshold_kernel<T, 4, 512, sizeof(T) == 4 ? 2 : 1>, rows, 512);   // bf16 would spill at two
+        } else {
+            if (n_samples <= 128 || n_qheads > (n_samples > 1024 ? 3 : 2) * SM_COUNT) run(threshold_kernel<T, 2, 256, 4>, rows, 256);
+            else if (n_qheads > SM_COUNT) run(threshold_kernel<T, 2, 512, 2>, rows, 512);
+            else run(threshold_kernel<T, 2, 1024, 1>, rows, 1024);
+        }
+    };
+    if (dtype == HIRA_BF16) sized(reinterpret_cast<const __nv_bfloat16*>(samples));
+    else sized(reinterpret_cast<const float*>(samples));
     if (e != cudaSuccess) {
         set_error("hira_threshold launch: %s", cudaGetErrorString(e));
         return HIRA_ERR_CUDA;

@@ -414,7 +414,7 @@ def merge_partials(part_o, part_ml, out=None, out_ml=None):
 
 
 def _check_rows(t: torch.Tensor, h: int, m: int, width: int, dtype: torch.dtype):
-    if t.shape != (h, m, width):
+    if t.numel() != h * m * width:
         raise ValueError(f"expected ({h}, {m}, {width}) rows, got {tuple(t.shape)}")
     assert t.is_contiguous() and t.dtype == dtype
 

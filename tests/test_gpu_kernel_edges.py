@@ -338,3 +338,13 @@ def test_staged_append_of_many_heads_matches_oracle(h, depth, bf, n, m):
         S.append(st, nk, nv)
         O.append(ox, nk, nv)
     assert_index_equal(st, ox, "many heads")
+
+
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 64), (torch.float32, 136), (torch.bfloat16, 200)])
+@pytest.mark.parametrize("hq", [148, 149, 296, 297, 444, 445])
+@pytest.mark.parametrize("s,k", [(128, 128), (129, 33), (300, 5)])
+def test_threshold_of_many_heads_matches_oracle(dtype, d, hq, s, k):
+    """Both sides of the head and sample counts at which the block size changes."""
+    samples, q = make_keys(1, s, d, 3, dtype), make_queries(hq, d, seed=4)
+    got = S.threshold(samples, q, L.HIRA_TAU_SAMPLE_MEAN_TOPK, k).cpu().numpy()
+    assert np.array_equal(got.view(np.uint32), np.asarray(O.threshold(samples, q, L.HIRA_TAU_SAMPLE_MEAN_TOPK, k), np.float32).view(np.uint32))
