@@ -284,8 +284,9 @@ __global__ void gather_centres_kernel(const T* __restrict__ points, long long p_
 // sorted by one warp in registers, but any of them can be anything up to all the points of a head (hubs, padding
 // rows, constant keys): ranges of more than SORT_WARP members go to a work list in pieces of SORT_CTA, a piece is
 // sorted by one CTA, and ranges of several pieces are merged MERGE_WAYS runs at a time by the whole GPU.
-// (A device-wide radix sort of (centre, distance) before: 5 or 6 passes of about 9 us whatever the size; 8 x 32,768
-// points in 1,024 centres each 65 -> 30 us, 8 x 4,096 points in 64 73 -> 22 us with all of the kernels around it.)
+// (A device-wide radix sort of (centre, distance) before: 5 or 6 passes of about 9 us whatever the size.  8 x 4,096
+// points in 64 centres, an iteration with all of the kernels around the sort: 73 -> 16 us; a build of 8 x 32,768
+// points, both levels: radix sort 101 us, this 22 with 25 of small kernels.)
 // ---------------------------------------------------------------------------
 constexpr int SORT_THREADS = 256, SORT_RANGES = SORT_THREADS / 32, SORT_WARP = 128, SORT_CTA = 4096;
 constexpr int SORT_PIECE_CTAS = 2 * SM_COUNT;   // CTAs of the sort that serve the work list
