@@ -315,11 +315,13 @@ class CUDAIndexer(BaseIndexer):
                 for t in (new_keys, new_values):      # allocated on another stream, consumed on this one
                     if t is not None and t.is_cuda:
                         t.record_stream(stream)
-                with torch.cuda.stream(stream):
-                    self._update(new_keys, new_values, scanned, home=cur)
-                    done = torch.cuda.Event()
+                done = torch.cuda.Event()
+                try:
+                    with torch.cuda.stream(stream):
+                        self._update(new_keys, new_values, scanned, home=cur)
+                finally:      # also for a refused update: an earlier one may still be running there
                     done.record(stream)
-                self._pending_append = done
+                    self._pending_append = done
                 return self
         return self._update(new_keys, new_values, scanned)
 

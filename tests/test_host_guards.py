@@ -151,9 +151,7 @@ class _FakeStream:
         self.log.append((self.name, "waits for", "event"))
 
 
-def test_growth_of_a_side_stream_update_runs_where_the_index_lives(monkeypatch):
-    """The old arrays are read, and the new ones allocated, on the stream whose memory they are."""
-    log = []
+def _fake_streams(monkeypatch, log):
     main, side = _FakeStream("main", log), _FakeStream("side", log)
     active = [main]
 
@@ -169,6 +167,13 @@ def test_growth_of_a_side_stream_update_runs_where_the_index_lives(monkeypatch):
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: active[-1])
     monkeypatch.setattr(torch.cuda, "stream", _On)
     monkeypatch.setattr(torch.cuda, "Event", lambda: SimpleNamespace(record=lambda s: log.append((s.name, "record"))))
+    return side, active
+
+
+def test_growth_of_a_side_stream_update_runs_where_the_index_lives(monkeypatch):
+    """The old arrays are read, and the new ones allocated, on the stream whose memory they are."""
+    log = []
+    side, active = _fake_streams(monkeypatch, log)
     grown = S.IndexState.grown
     monkeypatch.setattr(S.IndexState, "grown", lambda st, n: log.append((active[-1].name, "grows")) or grown(st, n))
     monkeypatch.setattr(S.IndexState, "used_on", lambda st, s: log.append((s.name, "uses", st.cap_parents)), raising=False)
@@ -264,3 +269,18 @@ def test_append_slices_fit_the_gpu_at_once(heads, cap, depth, parts):
     for m in (1, 32):
         assert L.load().hira_append_workspace_bytes(st.struct, m) == heads * m * (parts + 1) * 8
     assert L.load().hira_append_workspace_bytes(st.struct, 33) == 0
+
+
+def test_a_refused_side_stream_update_does_not_hide_the_one_before(monkeypatch):
+    log = []
+    side, active = _fake_streams(monkeypatch, log)
+    monkeypatch.setattr(S.IndexState, "used_on", lambda st, s: None)
+    monkeypatch.setattr(S, "append", lambda st, k, v: None)
+    ix = _indexer()
+    row = torch.zeros(1, 4, 1, 64, dtype=torch.bfloat16)
+    ix.update(row, row, stream=side)
+    with pytest.raises(ValueError):
+        ix.update(row[..., :32], row, stream=side)
+    log.clear()
+    ix.wait_pending_update()
+    assert log == [("main", "waits for", "event")]
